@@ -505,6 +505,7 @@ int exa_ctx_init(ExaCtx& c, const double* app, long long napp, const double* mas
   EXA_TRY(dev_alloc(c, &c.gcs, n1));
   EXA_TRY(dev_alloc(c, &c.gsn, n1));
   EXA_TRY(dev_alloc(c, &c.scal, 16));
+  EXA_TRY(dev_alloc(c, &c.ortho_work, exa_ortho_work(c.restart)));
   if (c.ppdegree > 1) {
     // start vector of the polynomial's Arnoldi process: seeded normal values on the trace
     // nodes, normalised (the reference draws rand() normals on the element nodes, averages

@@ -124,9 +124,6 @@ int exa_reduce_partials(const double* part, long long n, double* out, int take_s
 int exa_axpby(double* y, const double* x, double a, double b, long long n, cudaStream_t st);
 int exa_scale(double* y, const double* x, double a, long long n, cudaStream_t st);
 int exa_fill(double* y, double a, long long n, cudaStream_t st);
-// One modified Gram-Schmidt step: h = sum(part_in); w -= h * vprev; part_out = partial(w . vnext).
-int exa_mgs_step(double* w, const double* vprev, const double* vnext, const double* part_in,
-                 double* part_out, double* h_out, long long n, cudaStream_t st);
 // h = sqrt(sum(part_in)); v = w / h.
 int exa_mgs_finish(double* v, const double* w, const double* part_in, double* h_out, long long n,
                    cudaStream_t st);
@@ -134,6 +131,24 @@ int exa_mgs_finish(double* v, const double* w, const double* part_in, double* h_
 // |s[i+1]| / nrmb to *relerr.
 int exa_givens(double* hcol, double* s, double* cs, double* sn, int i, const double* nrmb,
                double* relerr, cudaStream_t st);
+// The Givens state of a GMRES cycle: rotations cs, sn and the rotated right-hand side s, the norm
+// the residual estimate is relative to, and where the estimate goes (device and mapped host
+// memory).  inv is exa_mgs's own.
+struct ExaGivens {
+  double *s, *cs, *sn;
+  const double* nrmb;
+  double *rel, *rel_host, *inv;
+};
+// Modified Gram-Schmidt of w against the k columns of V (exa_ortho.cu): hcol(0:k) = the
+// coefficients, hcol(k) = the norm of what is left, w <- that, normalised.  With givens, the
+// rotations of Hessenberg column k - 1 follow (cpuApplyGivensRotation semantics) and the residual
+// estimate goes to givens->rel and givens->rel_host.  The columns of V must have come from this
+// routine in order (column k - 1 newest): work, exa_ortho_work(restart) doubles that start zeroed,
+// holds their products from call to call.
+constexpr int EXA_ORTHO_PANEL = 64, EXA_ORTHO_BLOCKS = 296;
+size_t exa_ortho_work(int restart);
+int exa_mgs(double* w, const double* V, long long n, int k, double* hcol, double* work, int restart,
+            const ExaGivens* givens, cudaStream_t st);
 // x += V(:, 0:k) y   (V column-major N x k, y on device)
 int exa_gemv_add(double* x, const double* V, const double* y, long long n, int k, cudaStream_t st);
 // hcol(0:k) = V(:, 0:k)^T w, then w -= V(:,0:k) hcol(0:k)   (classical Gram-Schmidt)

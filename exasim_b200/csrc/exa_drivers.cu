@@ -270,23 +270,6 @@ int apply_poly(ExaCtx& c, double* wv) {
   return EXA_OK;
 }
 
-// v_j <- v_j orthogonalised against v_0 .. v_{j-1} by modified Gram-Schmidt and normalised,
-// the coefficients into hcol[0 .. j] (MGS, getpoly.cpp:36-45; the pipelined launches of
-// arnoldi_ops)
-int mgs_column(ExaCtx& c, int j, double* hcol) {
-  const long long N = c.sysN();
-  double* vn = c.V + (long long)j * N;
-  EXA_TRY(exa_dot_partials(vn, c.V, N, c.part_a, c.st));
-  double* pin = c.part_a;
-  double* pout = c.part_b;
-  for (int k = 1; k < j; ++k) {
-    EXA_TRY(exa_mgs_step(vn, c.V + (long long)(k - 1) * N, c.V + (long long)k * N, pin, pout, hcol + k - 1, N, c.st));
-    std::swap(pin, pout);
-  }
-  EXA_TRY(exa_mgs_step(vn, c.V + (long long)(j - 1) * N, nullptr, pin, pout, hcol + j - 1, N, c.st));
-  return exa_mgs_finish(vn, vn, pout, hcol + j, N, c.st);
-}
-
 // getPoly (getpoly.cpp:226-247) and the Ritz-value post-processing of GMRES (gmres.cpp:385-398):
 // m = ppdegree Arnoldi steps of P A from randvect (makeH, getpoly.cpp:208-224), then on the
 // host the harmonic Ritz values in Leja order (exa_poly_ritz)
@@ -298,7 +281,8 @@ int poly_setup(ExaCtx& c) {
   EXA_TRY(exa_scale(c.V, c.randvect, 1.0 / nr, N, c.st));
   for (int j = 0; j < m; ++j) {
     EXA_TRY(pa(c, c.V + (long long)j * N, c.V + (long long)(j + 1) * N));
-    EXA_TRY(mgs_column(c, j + 1, c.hess + (long long)n1 * j));
+    EXA_TRY(exa_mgs(c.V + (long long)(j + 1) * N, c.V, N, j + 1, c.hess + (long long)n1 * j, c.ortho_work, c.restart,
+                    nullptr, c.st));
   }
   EXA_CUDA(cudaMemcpyAsync(c.pinned, c.hess, sizeof(double) * n1 * m, cudaMemcpyDeviceToHost, c.st));
   EXA_CUDA(cudaStreamSynchronize(c.st));
@@ -339,20 +323,13 @@ int arnoldi_ops(ExaCtx& c, int i, const double* d_nrmb, double* d_relerr, double
   {
     ExaProfScope ps_ortho(c, EXA_PH_ORTHO);
     if (c.ortho == 0) {
-      EXA_TRY(exa_dot_partials(vn, c.V, N, c.part_a, c.st));
-      double* pin = c.part_a;
-      double* pout = c.part_b;
-      for (int k = 1; k <= i; ++k) {
-        EXA_TRY(exa_mgs_step(vn, c.V + (long long)(k - 1) * N, c.V + (long long)k * N, pin, pout, hcol + k - 1, N, c.st));
-        std::swap(pin, pout);
-      }
-      EXA_TRY(exa_mgs_step(vn, c.V + (long long)i * N, nullptr, pin, pout, hcol + i, N, c.st));
-      EXA_TRY(exa_mgs_finish(vn, vn, pout, hcol + i + 1, N, c.st));
-    } else {
-      EXA_TRY(exa_cgs(vn, c.V, hcol, c.part_m, N, i + 1, c.st));
-      EXA_TRY(exa_dot_partials(vn, vn, N, c.part_a, c.st));
-      EXA_TRY(exa_mgs_finish(vn, vn, c.part_a, hcol + i + 1, N, c.st));
+      // with the Givens update of the column; the residual estimate goes straight to the slot
+      const ExaGivens g{c.gs, c.gcs, c.gsn, d_nrmb, d_relerr, rel_pin, nullptr};
+      return exa_mgs(vn, c.V, N, i + 1, hcol, c.ortho_work, c.restart, &g, c.st);
     }
+    EXA_TRY(exa_cgs(vn, c.V, hcol, c.part_m, N, i + 1, c.st));
+    EXA_TRY(exa_dot_partials(vn, vn, N, c.part_a, c.st));
+    EXA_TRY(exa_mgs_finish(vn, vn, c.part_a, hcol + i + 1, N, c.st));
   }
   EXA_TRY(exa_givens(hcol, c.gs, c.gcs, c.gsn, i, d_nrmb, d_relerr, c.st));
   EXA_CUDA(cudaMemcpyAsync(rel_pin, d_relerr, sizeof(double), cudaMemcpyDeviceToHost, c.st));

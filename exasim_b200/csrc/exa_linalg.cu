@@ -1280,42 +1280,6 @@ __global__ void fill_kernel(double* y, double a, long long n) {
     y[i] = a;
 }
 
-__global__ void __launch_bounds__(VT) mgs_step_kernel(double* w, const double* vprev, const double* vnext,
-                                                      const double* part_in, double* part_out, double* h_out,
-                                                      long long n) {
-  const double h = sum_partials_n(part_in, gridDim.x);
-  if (blockIdx.x == 0 && threadIdx.x == 0) *h_out = h;
-  double v = 0.0;
-  // the basis vectors stream through (evict-first loads), so a vector being orthogonalised
-  // that fits in L2 stays there across the steps of its Gram-Schmidt sweep.  Four strides'
-  // loads are issued before their updates (long vectors need the loads in flight); the
-  // products are summed in the same order as one stride at a time.
-  const long long stride = (long long)gridDim.x * VT;
-  long long i = blockIdx.x * (long long)VT + threadIdx.x;
-  for (; i + 3 * stride < n; i += 4 * stride) {
-    double ww[4], p[4], q[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      ww[u] = w[i + u * stride];
-      p[u] = __ldcs(vprev + i + u * stride);
-      q[u] = vnext ? __ldcs(vnext + i + u * stride) : 0.0;
-    }
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const double wi = ww[u] - h * p[u];
-      w[i + u * stride] = wi;
-      v = fma(wi, vnext ? q[u] : wi, v);
-    }
-  }
-  for (; i < n; i += stride) {
-    double wi = w[i] - h * __ldcs(vprev + i);
-    w[i] = wi;
-    v = fma(wi, vnext ? __ldcs(vnext + i) : wi, v);
-  }
-  double s = block_sum(v);
-  if (threadIdx.x == 0) part_out[blockIdx.x] = s;
-}
-
 __global__ void __launch_bounds__(VT) mgs_finish_kernel(double* vout, const double* w, const double* part_in,
                                                         double* h_out, long long n) {
   const double h = sqrt(sum_partials_n(part_in, gridDim.x));
@@ -1359,14 +1323,6 @@ __global__ void givens_kernel(double* H, double* s, double* cs, double* sn, int 
   H[i] = cs[i] * H[i] + sn[i] * H[i + 1];
   H[i + 1] = 0.0;
   *relerr = fabs(s[i + 1]) / *nrmb;
-}
-
-__global__ void gemv_add_kernel(double* x, const double* V, const double* y, long long n, int k) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    double acc = 0.0;
-    for (int j = 0; j < k; ++j) acc = fma(V[i + n * j], y[j], acc);
-    x[i] += acc;
-  }
 }
 
 // partial dots of w against the k columns of V: part[j*VB + block]
@@ -1432,13 +1388,6 @@ int exa_fill(double* y, double a, long long n, cudaStream_t st) {
   return EXA_OK;
 }
 
-int exa_mgs_step(double* w, const double* vprev, const double* vnext, const double* part_in,
-                 double* part_out, double* h_out, long long n, cudaStream_t st) {
-  mgs_step_kernel<<<vec_grid(n), VT, 0, st>>>(w, vprev, vnext, part_in, part_out, h_out, n);
-  EXA_LAUNCH_CHECK();
-  return EXA_OK;
-}
-
 int exa_mgs_finish(double* v, const double* w, const double* part_in, double* h_out, long long n, cudaStream_t st) {
   mgs_finish_kernel<<<vec_grid(n), VT, 0, st>>>(v, w, part_in, h_out, n);
   EXA_LAUNCH_CHECK();
@@ -1448,13 +1397,6 @@ int exa_mgs_finish(double* v, const double* w, const double* part_in, double* h_
 int exa_givens(double* hcol, double* s, double* cs, double* sn, int i, const double* nrmb, double* relerr,
                cudaStream_t st) {
   givens_kernel<<<1, 1, 0, st>>>(hcol, s, cs, sn, i, nrmb, relerr);
-  EXA_LAUNCH_CHECK();
-  return EXA_OK;
-}
-
-int exa_gemv_add(double* x, const double* V, const double* y, long long n, int k, cudaStream_t st) {
-  if (k <= 0) return EXA_OK;
-  gemv_add_kernel<<<vec_grid(n), VT, 0, st>>>(x, V, y, n, k);
   EXA_LAUNCH_CHECK();
   return EXA_OK;
 }

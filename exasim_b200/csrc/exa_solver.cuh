@@ -69,7 +69,7 @@ struct ExaCtx {
   // Krylov / Newton workspace
   double *V = nullptr, *x = nullptr, *r = nullptr, *w = nullptr, *we = nullptr, *du = nullptr;
   double *part_a = nullptr, *part_b = nullptr, *part_m = nullptr, *hess = nullptr, *gs = nullptr, *gcs = nullptr,
-         *gsn = nullptr, *scal = nullptr, *udgprev = nullptr, *utmp = nullptr;
+         *gsn = nullptr, *scal = nullptr, *ortho_work = nullptr, *udgprev = nullptr, *utmp = nullptr;
   int* d_flag = nullptr;
   double* pinned = nullptr;  // small host staging buffer
   // reduced-basis initial guess of GMRES (RBdim > 0): the last RBdim Newton updates W, their
