@@ -298,7 +298,7 @@ int exa_ctx_init(ExaCtx& c, const double* app, long long napp, const double* mas
       return EXA_ERR_UNSUPPORTED;
     }
     const int ncf = P.ncu * P.npf;
-    if (ncf > 64 || exa_bilu_apply_smem(ncf, hb.nfse) > 227 * 1024) {
+    if (ncf > 64 || !exa_bilu_fits(ncf, hb.nfse)) {
       exa_set_error("block ILU(0): %d faces of %d rows per sub-domain exceed shared memory", hb.nfse, ncf);
       return EXA_ERR_UNSUPPORTED;
     }
@@ -313,6 +313,15 @@ int exa_ctx_init(ExaCtx& c, const double* app, long long napp, const double* mas
     EXA_TRY(dev_upload(c, &d.upd_ptr, hb.upd_ptr.data(), hb.upd_ptr.size()));
     EXA_TRY(dev_upload(c, &d.upd_jl, hb.upd_jl.data(), std::max<size_t>(1, hb.upd_jl.size())));
     EXA_TRY(dev_upload(c, &d.upd_il, hb.upd_il.data(), std::max<size_t>(1, hb.upd_il.size())));
+    for (int up = 0; up < 2; ++up) {
+      const ExaSweep& h = up ? hb.bwd : hb.fwd;
+      ExaSweepDev& w = up ? d.bwd : d.fwd;
+      w.levels = (int)h.lev.size() - 1;
+      EXA_TRY(dev_upload(c, &w.lev, h.lev.data(), h.lev.size()));
+      EXA_TRY(dev_upload(c, &w.row, h.row.data(), std::max<size_t>(1, h.row.size())));
+      EXA_TRY(dev_upload(c, &w.ptr, h.ptr.data(), h.ptr.size()));
+      EXA_TRY(dev_upload(c, &w.blk, h.blk.data(), std::max<size_t>(1, h.blk.size())));
+    }
     EXA_TRY(dev_upload(c, &d.gf_ptr, hb.gf_ptr.data(), hb.gf_ptr.size()));
     EXA_TRY(dev_upload(c, &d.gf_pos, hb.gf_pos.data(), hb.gf_pos.size()));
     EXA_TRY(dev_alloc(c, &d.out, (size_t)hb.nse * hb.nfse * ncf));

@@ -252,6 +252,36 @@ int exa_bilu_setup(const int* cgp, int ncgp, const int* f2e_in, int nf, int nfe,
     }
     b.fac_ptr.push_back((int)b.fac_ji.size());
   }
+  // ---- levels of the two sweeps: row i of L waits for its columns j < i, of U for l > i
+  for (int up = 0; up < 2; ++up) {
+    ExaSweep& w = up ? b.bwd : b.fwd;
+    Vec level(nfs, 0);
+    int nlev = 0;
+    for (int q = 0; q < nfs; ++q) {
+      const int i = up ? nfs - 1 - q : q;
+      for (int t = b.row_ptr[i] + 1; t < b.row_ptr[i + 1]; ++t)
+        if ((b.col_ind[t] > i) == (up == 1)) level[i] = std::max(level[i], level[b.col_ind[t]] + 1);
+      nlev = std::max(nlev, level[i] + 1);
+    }
+    w.lev.assign(1, 0);
+    w.ptr.assign(1, 0);
+    for (int l = 0; l < nlev; ++l) {
+      for (int i = 0; i < nfs; ++i) {
+        if (level[i] != l) continue;
+        Vec deps;
+        for (int t = b.row_ptr[i] + 1; t < b.row_ptr[i + 1]; ++t)
+          if ((b.col_ind[t] > i) == (up == 1)) deps.push_back(t);
+        if (!up && deps.empty()) continue;  // L has unit diagonal blocks: nothing to do
+        const int r0 = w.lev.back(), nr = (int)w.row.size() - r0;
+        if (nr == ExaSweep::kRows || (nr > 0 && w.ptr.back() - w.ptr[r0] + (int)deps.size() > ExaSweep::kBlks))
+          w.lev.push_back((int)w.row.size());
+        w.row.push_back(i);
+        w.blk.insert(w.blk.end(), deps.begin(), deps.end());
+        w.ptr.push_back((int)w.blk.size());
+      }
+      if ((int)w.row.size() > w.lev.back()) w.lev.push_back((int)w.row.size());
+    }
+  }
   // ---- summing back: copies of each global face in fixed (sub-domain, local face) order
   std::vector<Vec> copies(nf);
   for (int i = 0; i < nfs; ++i)

@@ -5,10 +5,11 @@
 // Blocks are ncf x ncf (ncf = ncu npf), column-major; block (r, t) of sub-domain r and CRS
 // position t lies at BE + ncf^2 (r + nse t), as in the reference (kokkosimpl.h:1264-1341).
 // The factorization (matvec.cpp:119-166) and the sweeps (preconditioner.cpp:184-271) are
-// sequential over the faces of a sub-domain and parallel over the sub-domains: one CTA per
-// sub-domain walks the schedule built on the host (exa_bilu0.cpp) with dense block work
-// spread over its threads in shared memory.  The sub-domain results are summed back onto the
+// ordered over the faces of a sub-domain and parallel over the sub-domains: one CTA per
+// sub-domain walks the schedule built on the host (exa_bilu0.cpp; the sweeps by levels of
+// independent faces) with dense block work spread over its threads in shared memory.  The sub-domain results are summed back onto the
 // global faces in a fixed order (preconditioner.cpp:296-325 sums them atomically).
+#include "exa_bilu0.h"
 #include "exa_kernels.cuh"
 
 namespace {
@@ -166,71 +167,80 @@ __global__ void __launch_bounds__(256) bilu_factor_kernel(int ncf, int nse, int 
   }
 }
 
-// y = L^-1 (gathered x), z = U^-1 y per sub-domain; out[(r + nse i) ncf + a] = z_i[a]
+// row of a block times a vector in shared memory: 16 loads in flight (a row's blocks come from
+// L2), the sum in the order of the columns
 template <typename T>
-__global__ void __launch_bounds__(256) bilu_apply_kernel(int ncf, int nse, int nfse, const int* row_ptr,
-                                                         const int* col_ind, const int* face, const T* BE,
-                                                         const double* x, double* out) {
+__device__ __forceinline__ double block_row(const T* A, int ncf, const double* v) {
+  double s = 0.0;
+  for (int k0 = 0; k0 < ncf; k0 += 16) {
+    T t[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) t[u] = k0 + u < ncf ? A[ncf * (k0 + u)] : T(0);
+#pragma unroll
+    for (int u = 0; u < 16; ++u)
+      if (k0 + u < ncf) s = fma((double)t[u], v[k0 + u], s);
+  }
+  return s;
+}
+
+// y = L^-1 (gathered x), then y = U^-1 y in place, per sub-domain; out[(r + nse i) ncf + a] = y_i[a].
+//
+// Bound: the chain of dependent rows.  The sweeps go by levels of independent rows (9 each way for
+// 4 x 4 quadrilaterals against 40 rows): one thread per (block, row) of a level, then one per
+// (row, entry) adds the level's products in row order, so a level costs two or three barriers and
+// one round of loads in flight together.
+template <typename T>
+__global__ void __launch_bounds__(512) bilu_apply_kernel(int ncf, int nse, int nfse, const int* row_ptr,
+                                                         const int* col_ind, const int* face, ExaSweepDev L,
+                                                         ExaSweepDev U, const T* BE, const double* x, double* out) {
   extern __shared__ double asm_[];
-  double* y = asm_;                  // [nfse, ncf]
-  double* z = y + nfse * ncf;        // [nfse, ncf]
-  const int G = blockDim.x / ncf;    // groups of ncf threads share the blocks of a row
-  double* part = z + nfse * ncf;     // [G, ncf]
-  double* v = part + G * ncf;        // [ncf]
+  double* y = asm_;                            // [nfse, ncf]
+  double* part = y + nfse * ncf;               // [kBlks, ncf]: products of the level's blocks
+  double* v = part + ExaSweep::kBlks * ncf;    // [kRows, ncf]: right-hand sides of its rows
   const int r = blockIdx.x, nn = ncf * ncf;
-  const int a = threadIdx.x % ncf, g = threadIdx.x / ncf;
   auto blk = [&](int t) { return BE + (long long)nn * (r + (long long)nse * t); };
   for (int t = threadIdx.x; t < nfse * ncf; t += blockDim.x) {
     const int i = t / ncf, c = t % ncf;
     y[t] = x[(long long)ncf * face[r + nse * i] + c];
   }
   __syncthreads();
-  for (int i = 0; i < nfse; ++i) {
-    double s = 0.0;
-    if (g < G)
-      for (int t = row_ptr[i] + 1 + g; t < row_ptr[i + 1]; t += G) {
-        const int j = col_ind[t];
-        if (j >= i) continue;
-        const T* L = blk(t);
-        for (int k = 0; k < ncf; ++k) s += (double)L[a + ncf * k] * y[j * ncf + k];
-      }
-    if (g < G) part[g * ncf + a] = s;
+  auto products = [&](const ExaSweepDev& S, int b0, int b1) {
+    for (int t = threadIdx.x; t < (b1 - b0) * ncf; t += blockDim.x) {
+      const int q = t / ncf, a = t - q * ncf, p = S.blk[b0 + q];
+      part[t] = block_row(blk(p) + a, ncf, y + col_ind[p] * ncf);
+    }
     __syncthreads();
-    if (threadIdx.x < ncf) {
-      double acc = 0.0;
-      for (int q = 0; q < G; ++q) acc += part[q * ncf + threadIdx.x];
-      y[i * ncf + threadIdx.x] -= acc;
+  };
+  for (int l = 0; l < L.levels; ++l) {
+    const int r0 = L.lev[l], r1 = L.lev[l + 1], b0 = L.ptr[r0];
+    products(L, b0, L.ptr[r1]);
+    for (int t = threadIdx.x; t < (r1 - r0) * ncf; t += blockDim.x) {
+      const int q = r0 + t / ncf, a = t % ncf;
+      double s = 0.0;
+      for (int p = L.ptr[q]; p < L.ptr[q + 1]; ++p) s += part[(p - b0) * ncf + a];
+      y[L.row[q] * ncf + a] -= s;
     }
     __syncthreads();
   }
-  for (int i = nfse - 1; i >= 0; --i) {
-    double s = 0.0;
-    if (g < G)
-      for (int t = row_ptr[i] + 1 + g; t < row_ptr[i + 1]; t += G) {
-        const int l = col_ind[t];
-        if (l <= i) continue;
-        const T* U = blk(t);
-        for (int k = 0; k < ncf; ++k) s += (double)U[a + ncf * k] * z[l * ncf + k];
-      }
-    if (g < G) part[g * ncf + a] = s;
-    __syncthreads();
-    if (threadIdx.x < ncf) {
-      double acc = 0.0;
-      for (int q = 0; q < G; ++q) acc += part[q * ncf + threadIdx.x];
-      v[threadIdx.x] = y[i * ncf + threadIdx.x] - acc;
+  for (int l = 0; l < U.levels; ++l) {
+    const int r0 = U.lev[l], r1 = U.lev[l + 1], b0 = U.ptr[r0];
+    products(U, b0, U.ptr[r1]);
+    for (int t = threadIdx.x; t < (r1 - r0) * ncf; t += blockDim.x) {
+      const int q = r0 + t / ncf, a = t % ncf;
+      double s = 0.0;
+      for (int p = U.ptr[q]; p < U.ptr[q + 1]; ++p) s += part[(p - b0) * ncf + a];
+      v[t] = y[U.row[q] * ncf + a] - s;
     }
     __syncthreads();
-    if (threadIdx.x < ncf) {
-      const T* Di = blk(row_ptr[i]);
-      double acc = 0.0;
-      for (int k = 0; k < ncf; ++k) acc += (double)Di[threadIdx.x + ncf * k] * v[k];
-      z[i * ncf + threadIdx.x] = acc;
+    for (int t = threadIdx.x; t < (r1 - r0) * ncf; t += blockDim.x) {
+      const int q = t / ncf, a = t - q * ncf, i = U.row[r0 + q];
+      y[i * ncf + a] = block_row(blk(row_ptr[i]) + a, ncf, v + q * ncf);
     }
     __syncthreads();
   }
   for (int t = threadIdx.x; t < nfse * ncf; t += blockDim.x) {
     const int i = t / ncf, c = t % ncf;
-    out[((long long)r + (long long)nse * i) * ncf + c] = z[t];
+    out[((long long)r + (long long)nse * i) * ncf + c] = y[t];
   }
 }
 
@@ -255,9 +265,9 @@ int grid_of(long long n) {
 
 }  // namespace
 
-size_t exa_bilu_apply_smem(int ncf, int nfse) {
-  const int G = 256 / ncf;
-  return sizeof(double) * ((size_t)2 * nfse * ncf + (size_t)G * ncf + ncf);
+// two copies of a sub-domain's vector and a few rows fit in shared memory
+bool exa_bilu_fits(int ncf, int nfse) {
+  return sizeof(double) * ((size_t)2 * nfse * ncf + (size_t)(256 / ncf) * ncf + ncf) <= 227 * 1024;
 }
 
 template <typename T>
@@ -284,9 +294,11 @@ template <typename T>
 int exa_k_bilu_apply(const ExaDims& P, const ExaBiluDev& b, const T* BE, const double* x, double* w,
                      cudaStream_t st) {
   const int ncf = P.ncu * P.npf;
-  const size_t smem = exa_bilu_apply_smem(ncf, b.nfse);
+  // at ncf = 64, the largest, the buffers take 82 KB beside at most 114 KB of y (exa_bilu_fits)
+  const size_t smem = sizeof(double) * ncf * ((size_t)b.nfse + ExaSweep::kBlks + ExaSweep::kRows);
   EXA_TRY(exa_allow_smem((const void*)bilu_apply_kernel<T>, smem));
-  bilu_apply_kernel<T><<<b.nse, 256, smem, st>>>(ncf, b.nse, b.nfse, b.row_ptr, b.col_ind, b.face, BE, x, b.out);
+  bilu_apply_kernel<T><<<b.nse, 512, smem, st>>>(ncf, b.nse, b.nfse, b.row_ptr, b.col_ind, b.face, b.fwd, b.bwd, BE, x,
+                                                 b.out);
   EXA_LAUNCH_CHECK();
   bilu_sum_kernel<<<grid_of((long long)ncf * P.nf), 256, 0, st>>>(ncf, P.nf, b.gf_ptr, b.gf_pos, b.out, w);
   EXA_LAUNCH_CHECK();

@@ -47,14 +47,20 @@ int exa_k_vol_mat_tc(const ExaDims& P, const float* shapegw32, const UPacked& Sp
                      double* B, const UPacked& Bp, int nb, int* flag, cudaStream_t st);
 // Block ILU(0) preconditioner on Cartesian sub-domains (Exasim preconditioner = 2): the
 // schedule built on the host (exa_bilu0.h) in device memory, and the sub-domain results.
+struct ExaSweepDev {
+  int levels = 0;
+  int *lev = nullptr, *row = nullptr, *ptr = nullptr, *blk = nullptr;
+};
 struct ExaBiluDev {
   int nse = 0, nfse = 0, nnz = 0;
   int *row_ptr = nullptr, *col_ind = nullptr, *face = nullptr, *row_of = nullptr;
   int *fac_ptr = nullptr, *fac_ji = nullptr, *upd_ptr = nullptr, *upd_jl = nullptr, *upd_il = nullptr;
   int *gf_ptr = nullptr, *gf_pos = nullptr;
   double* out = nullptr;  // [nse * nfse, ncf]
+  ExaSweepDev fwd, bwd;   // the levels of the L and U sweeps
 };
-size_t exa_bilu_apply_smem(int ncf, int nfse);
+// whether sub-domains of nfse faces of ncf rows are supported
+bool exa_bilu_fits(int ncf, int nfse);
 // blocks from the condensed element matrices H, then the block ILU(0) in place
 template <typename T>
 int exa_k_bilu_build(const ExaDims& P, const ExaBiluDev& b, const int* f2e, const int* elemcon, const T* H, T* BE,
