@@ -109,6 +109,39 @@ int init_solution(ExaCtx& c, const Blob& S) {
 
 }  // namespace
 
+// The 1D tables of the master element when its shape tables are their Kronecker products to
+// rounding (quadrilaterals and hexahedra with as many Gauss points as nodes per dimension); the
+// file's own 1D tables (parts shap1dgt and gw1d) are checked against every table used.
+void find_tensor(ExaTensor& t, const Blob& M, const ExaDims& P, int elemtype) {
+  t.n1 = 0;
+  if (elemtype != 1 || P.nd < 2 || P.nd > 3 || M.nsize.size() < 22) return;
+  int n1 = 1;
+  while ((P.nd == 3 ? n1 * n1 * n1 : n1 * n1) < P.npe) ++n1;
+  const int np = P.nd == 3 ? n1 * n1 * n1 : n1 * n1, nf = np / n1;
+  if (n1 > EXA_TP_MAX || np != P.npe || P.nge != np || P.npf != nf || P.ngf != nf) return;
+  if (M.nsize[15] != 2LL * n1 * n1 || M.nsize[21] != n1) return;
+  for (int q = 0; q < n1 * n1; ++q) t.S[q] = M.part[15][q], t.D[q] = M.part[15][n1 * n1 + q];
+  for (int g = 0; g < n1; ++g) t.w[g] = M.part[21][g];
+  // tables [rows, cols, 1 + dims]: to the points (g, a) and, weighted, back (a, g)
+  auto matches = [&](const double* T, const double* W, int dims, int n) {
+    double big = 0.0, off = 0.0;
+    for (int d = 0; d <= dims; ++d)
+      for (int a = 0; a < n; ++a)
+        for (int g = 0; g < n; ++g) {
+          double v = 1.0, w = 1.0;
+          for (int r = 0, ga = g, aa = a; r < dims; ++r, ga /= n1, aa /= n1) {
+            v *= (d == r + 1 ? t.D : t.S)[ga % n1 + n1 * (aa % n1)];
+            w *= t.w[ga % n1];
+          }
+          const double tv = T[g + (size_t)n * (a + (size_t)n * d)], wv = W[a + (size_t)n * (g + (size_t)n * d)];
+          big = std::max(big, std::fabs(tv));
+          off = std::max(off, std::max(std::fabs(tv - v), std::fabs(wv - v * w)));
+        }
+    return off <= 1e-13 * big;
+  };
+  if (matches(M.part[1], M.part[2], P.nd, np) && matches(M.part[3], M.part[4], P.nd - 1, nf)) t.n1 = n1;
+}
+
 int exa_ctx_init(ExaCtx& c, const double* app, long long napp, const double* master, long long nmaster,
                  const double* mesh, long long nmesh, const double* sol, long long nsol, int device) {
   Blob A = split_blob(app, napp), M = split_blob(master, nmaster), Me = split_blob(mesh, nmesh),
@@ -356,6 +389,24 @@ int exa_ctx_init(ExaCtx& c, const double* app, long long napp, const double* mas
     }
     EXA_TRY(dev_alloc(c, &c.ldg_fcon, 2 * (size_t)P.npf * P.nf));
     EXA_TRY(exa_k_ldg_fcon(P, c.f2e, c.perm, c.elemcon, c.ldg_fcon, c.st));
+    // tensor-product elements: the tables of the element kernel (every node on at most nd faces)
+    find_tensor(c.tensor, M, P, c.elemtype);
+    if (c.tensor.n1 > 0 && c.ldg_split && (long long)P.npf * P.ncu * P.nf < (1LL << 31)) {
+      std::vector<int> ns((size_t)P.nd * P.npe, -1);
+      bool ok = true;
+      for (int t = 0; t < P.ndf && ok; ++t) {
+        int* s = &ns[(size_t)P.nd * perm[t]];
+        int q = 0;
+        while (q < P.nd && s[q] >= 0) ++q;
+        ok = q < P.nd;
+        if (ok) s[q] = t;
+      }
+      if (ok) {
+        EXA_TRY(dev_upload(c, &c.ldg_nslot, ns.data(), ns.size()));
+        EXA_TRY(dev_alloc(c, &c.ldg_fslot, (size_t)P.ndf * P.ne));
+        EXA_TRY(exa_k_ldg_slots(P, c.f2e, c.elemcon, c.ldg_fslot, c.st));
+      }
+    }
     const size_t nl = (size_t)P.npe * P.ncu * ne;
     EXA_TRY(dev_alloc(c, &c.ldg_R, nl));
     EXA_TRY(dev_alloc(c, &c.ldg_w, nl));

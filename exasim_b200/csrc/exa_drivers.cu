@@ -158,11 +158,7 @@ int exa_drv_residual(ExaCtx& c, double* norm) {
 int ldg_matvec(ExaCtx& c, const double* v, double* w) {
   const long long N = c.sysN();
   const double eps = c.matvec_eps;
-  if (c.matvec_order == 1) {
-    EXA_TRY(exa_lincomb(c.ldg_w, 1.0, c.udg, eps, v, N, c.st));
-    EXA_TRY(exa_model_ldg_residual(c, c.ldg_w, c.ldg_Rw));
-    return exa_lincomb(w, 1.0 / eps, c.ldg_Rw, -1.0 / eps, c.ldg_R, N, c.st);
-  }
+  if (c.matvec_order == 1) return exa_model_ldg_jv(c, v, w);
   EXA_TRY(exa_lincomb(c.ldg_w, 1.0, c.udg, -eps, v, N, c.st));
   EXA_TRY(exa_model_ldg_residual(c, c.ldg_w, c.ldg_Rm));
   EXA_TRY(exa_lincomb(c.ldg_w, 1.0, c.udg, eps, v, N, c.st));

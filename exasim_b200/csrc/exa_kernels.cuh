@@ -47,6 +47,14 @@ int exa_k_vol_mat_tc(const ExaDims& P, const float* shapegw32, const UPacked& Sp
                      double* B, const UPacked& Bp, int nb, int* flag, cudaStream_t st);
 // Block ILU(0) preconditioner on Cartesian sub-domains (Exasim preconditioner = 2): the
 // schedule built on the host (exa_bilu0.h) in device memory, and the sub-domain results.
+// The 1D tables of a tensor-product element: its shape tables, and its faces', are Kronecker
+// products of S (and D for the derivatives) with the first dimension fastest, at n1 nodes and n1
+// Gauss points per dimension; n1 = 0 where they are not.
+constexpr int EXA_TP_MAX = 6;
+struct ExaTensor {
+  int n1 = 0;
+  double S[EXA_TP_MAX * EXA_TP_MAX], D[EXA_TP_MAX * EXA_TP_MAX], w[EXA_TP_MAX];  // S[g + n1 a]
+};
 struct ExaSweepDev {
   int levels = 0;
   int *lev = nullptr, *row = nullptr, *ptr = nullptr, *blk = nullptr;
@@ -92,6 +100,9 @@ int exa_k_face_nodes(const ExaDims& P, const int* f2e, const int* perm, const do
 // LDG (exa_ldg.cu): the face-node table of both sides [2, npf, nf]; the element residual from
 // the volume residual Rue and the face residuals Rh [npf, ncu, nf]; out = a x + b y
 int exa_k_ldg_fcon(const ExaDims& P, const int* f2e, const int* perm, const int* elemcon, int* fcon, cudaStream_t st);
+// slot[a + npf l + ndf e] = i + npf ncu f for node i of face f there, bit 31 set where the element
+// is the face's second one: where ldg_elem_tp_kernel finds the face residuals
+int exa_k_ldg_slots(const ExaDims& P, const int* f2e, const int* elemcon, int* slot, cudaStream_t st);
 int exa_k_ldg_gather(const ExaDims& P, const int* f2e, const int* perm, const int* elemcon, const double* Rue,
                      const double* Rh, double* Ru, int tdep, double dtfactor, cudaStream_t st);
 int exa_lincomb(double* out, double a, const double* x, double b, const double* y, long long n, cudaStream_t st);

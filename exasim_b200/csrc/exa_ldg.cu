@@ -31,6 +31,17 @@ __global__ void ldg_fcon_boundary_kernel(ExaDims P, const int* f2e, int* fcon) {
   }
 }
 
+__global__ void ldg_slots_kernel(ExaDims P, const int* f2e, const int* elemcon, int* slot) {
+  const long long total = (long long)P.ndf * P.ne;
+  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
+       t += (long long)gridDim.x * blockDim.x) {
+    const int jf = (int)(t % P.ndf), e = (int)(t / P.ndf), l = jf / P.npf;
+    const int g = elemcon[t], f = g / P.npf;
+    const bool first = f2e[4 * f] == e && f2e[4 * f + 1] == l;
+    slot[t] = (int)((unsigned)(g - f * P.npf + P.npf * P.ncu * f) | (first ? 0u : 0x80000000u));
+  }
+}
+
 // Ru of element e: its volume residual, minus the face residuals of the faces it is the first
 // element of and plus those of the others, face by face in the order of its local faces
 // (PutFaceNodes, kokkosimpl.h:1575-1603); then Ru <- -Ru and, time-dependent, Ru <- Ru / dtfactor
@@ -95,6 +106,12 @@ int exa_k_ldg_fcon(const ExaDims& P, const int* f2e, const int* perm, const int*
   ldg_fcon_kernel<<<blocks_for((long long)P.ndf * P.ne), 256, 0, st>>>(P, f2e, perm, elemcon, fcon);
   EXA_LAUNCH_CHECK();
   ldg_fcon_boundary_kernel<<<blocks_for((long long)P.npf * P.nf), 256, 0, st>>>(P, f2e, fcon);
+  EXA_LAUNCH_CHECK();
+  return EXA_OK;
+}
+
+int exa_k_ldg_slots(const ExaDims& P, const int* f2e, const int* elemcon, int* slot, cudaStream_t st) {
+  ldg_slots_kernel<<<blocks_for((long long)P.ndf * P.ne), 256, 0, st>>>(P, f2e, elemcon, slot);
   EXA_LAUNCH_CHECK();
   return EXA_OK;
 }

@@ -7,6 +7,7 @@
 
 #include "exa_assembly.cuh"
 #include "exa_ldg.cuh"
+#include "exa_ldg_tp.cuh"
 #include "exa_solver.cuh"
 #include "exa_umma.cuh"
 #include EXA_MODEL_HEADER
@@ -452,6 +453,48 @@ int exa_model_assemble(ExaCtx& c, bool jacobian) {
 
 bool exa_model_has_ldg_boundary() { return ExaModel::has_ldg_boundary; }
 
+namespace {
+
+LdgArgs ldg_args(const ExaCtx& c, const double* u) {
+  LdgArgs L{};
+  L.P = c.P;
+  L.shapfgt = c.shapfgt; L.shapfgw = c.shapfgw; L.shapfnt = c.shapfnt;
+  L.f2e = c.f2e; L.perm = c.perm; L.bf = c.bf; L.fcon = c.ldg_fcon;
+  L.xdg = c.xdg; L.faceg = c.faceg; L.uinf = c.uinf; L.param = c.param; L.tau = c.tau;
+  L.ntau = c.ntau; L.modelnumber = c.modelnumber; L.time = c.time;
+  L.u = u; L.Rh = c.ldg_Rh;
+  return L;
+}
+
+// the general face kernel over faces f0 .. nf - 1
+int ldg_faces_general(const ExaCtx& c, LdgArgs L, int f0) {
+  if (c.P.nf <= f0) return EXA_OK;
+  const size_t fs = ldg_face_smem(c.P);
+  EXA_TRY(smem_attr((const void*)ldg_face_kernel<ExaModel>, fs));
+  L.f0 = f0;
+  ldg_face_kernel<ExaModel><<<c.P.nf - f0, 64, fs, c.st>>>(L);
+  EXA_LAUNCH_CHECK();
+  return EXA_OK;
+}
+
+// out = U.cr R(u) + U.c0 U.R0 (or R(u)) by the tensor-product kernels; false where they do not apply.
+// Boundary faces take their states from L.u alone, so U.v is given on meshes without them only.
+bool ldg_residual_tp(ExaCtx& c, const LdgState& U, double* out, int* rc) {
+  if (!c.ldg_fslot || !c.ldg_split) return false;
+  struct Boundary {
+    ExaCtx& c;
+    LdgArgs L;
+  } b{c, ldg_args(c, U.u)};
+  auto boundary = [](void* p) -> int {
+    Boundary& q = *static_cast<Boundary*>(p);
+    return ldg_faces_general(q.c, q.L, q.c.P.nf0);
+  };
+  return launch_ldg_tp<ExaModel>(b.L, make_args(c, 0), U, c.tensor, c.ldg_nslot, c.ldg_fslot, out, c.st, boundary, &b,
+                                 rc);
+}
+
+}  // namespace
+
 // The LDG residual of the element states u (the layout of udg: nc = ncu without q): the volume
 // integrals of the HDG residual (RuElem, uresidual.cpp:45-130, is the same quadrature), the
 // face residuals of every face, and their sum into the elements with the sign and scaling of
@@ -459,6 +502,8 @@ bool exa_model_has_ldg_boundary() { return ExaModel::has_ldg_boundary; }
 int exa_model_ldg_residual(ExaCtx& c, const double* u, double* Ru) {
   const ExaDims& P = c.P;
   ExaProfScope ps(c, EXA_PH_RESIDUAL);
+  int rc = EXA_OK;
+  if (ldg_residual_tp(c, LdgState{u, nullptr, nullptr, 0.0, 1.0, 0.0}, Ru, &rc)) return rc;
   double* saved = c.udg;
   c.udg = const_cast<double*>(u);
   auto body = [&]() -> int {
@@ -475,15 +520,7 @@ int exa_model_ldg_residual(ExaCtx& c, const double* u, double* Ru) {
       EXA_LAUNCH_CHECK();
       if (c.wRG) EXA_TRY(volume_residual_gemm(c, Ruc, nb));
     }
-    LdgArgs L{};
-    L.P = P;
-    L.shapfgt = c.shapfgt; L.shapfgw = c.shapfgw; L.shapfnt = c.shapfnt;
-    L.f2e = c.f2e; L.perm = c.perm; L.bf = c.bf; L.fcon = c.ldg_fcon;
-    L.xdg = c.xdg; L.faceg = c.faceg; L.uinf = c.uinf; L.param = c.param; L.tau = c.tau;
-    L.ntau = c.ntau; L.modelnumber = c.modelnumber; L.time = c.time;
-    L.u = u; L.Rh = c.ldg_Rh;
-    const size_t fs = ldg_face_smem(P);
-    EXA_TRY(smem_attr((const void*)ldg_face_kernel<ExaModel>, fs));
+    LdgArgs L = ldg_args(c, u);
     // interior faces by the pointwise kernel where the model's (nd, ncu) has one, the boundary
     // faces (and otherwise all) by the general one
     int fgen = 0;
@@ -491,16 +528,32 @@ int exa_model_ldg_residual(ExaCtx& c, const double* u, double* Ru) {
       EXA_LAUNCH_CHECK();
       fgen = P.nf0;
     }
-    if (P.nf > fgen) {
-      L.f0 = fgen;
-      ldg_face_kernel<ExaModel><<<P.nf - fgen, 64, fs, c.st>>>(L);
-      EXA_LAUNCH_CHECK();
-    }
+    EXA_TRY(ldg_faces_general(c, L, fgen));
     return exa_k_ldg_gather(P, c.f2e, c.perm, c.elemcon, c.Ru, c.ldg_Rh, Ru, c.tdep, c.dtfactor, c.st);
   };
   const int st = body();
   c.udg = saved;
   return st;
+}
+
+int exa_model_ldg_jv(ExaCtx& c, const double* v, double* w) {
+  const long long N = c.sysN();
+  const double eps = c.matvec_eps;
+  const bool bnd = c.P.nf > c.P.nf0;
+  if (bnd) EXA_TRY(exa_lincomb(c.ldg_w, 1.0, c.udg, eps, v, N, c.st));
+  {
+    ExaProfScope ps(c, EXA_PH_RESIDUAL);
+    LdgState U{c.udg, v, c.ldg_R, eps, 1.0 / eps, -1.0 / eps};
+    if (bnd) {
+      U.u = c.ldg_w;
+      U.v = nullptr;
+    }
+    int rc = EXA_OK;
+    if (ldg_residual_tp(c, U, w, &rc)) return rc;
+  }
+  if (!bnd) EXA_TRY(exa_lincomb(c.ldg_w, 1.0, c.udg, eps, v, N, c.st));
+  EXA_TRY(exa_model_ldg_residual(c, c.ldg_w, c.ldg_Rw));
+  return exa_lincomb(w, 1.0 / eps, c.ldg_Rw, -1.0 / eps, c.ldg_R, N, c.st);
 }
 
 // initial u from the model's cpuInitu at the element nodes (readsolstruct, readbinaryfiles.cpp:546-556)

@@ -142,6 +142,10 @@ struct ExaCtx {
   // R(u), a perturbed state, its residual, the face residuals [npf, ncu, nf], R at u - eps v
   double *ldg_R = nullptr, *ldg_w = nullptr, *ldg_Rw = nullptr, *ldg_Rh = nullptr, *ldg_Rm = nullptr;
   int ldg_has_boundary = 0;
+  // tensor-product elements (n1 > 0): the 1D tables, and for the LDG element kernel the face
+  // slots of each node [npe, nd] (-1: none) and of each element's face nodes
+  ExaTensor tensor;
+  int *ldg_nslot = nullptr, *ldg_fslot = nullptr;
   // interior faces are faces [0, nf0) and boundary faces the rest (the pointwise interior-face
   // kernel relies on it)
   int ldg_split = 0;
@@ -169,6 +173,8 @@ int exa_model_assemble(ExaCtx& c, bool jacobian);
 int exa_model_init_udg(ExaCtx& c, double* host_udg);
 // LDG residual (residual.cpp:589-617) of the element states u [npe, ncu, ne] into Ru
 int exa_model_ldg_residual(ExaCtx& c, const double* u, double* Ru);
+// w = (R(u + eps v) - R(u)) / eps around u = udg with R(u) in ldg_R (one-sided differences)
+int exa_model_ldg_jv(ExaCtx& c, const double* v, double* w);
 // whether the model carries the LDG boundary functions (Ubou, Fbou)
 bool exa_model_has_ldg_boundary();
 
