@@ -90,49 +90,62 @@ __global__ void gemv_batch_kernel(GemmBatch g) {
 }
 
 // ----------------------------------------------------------------------------------
-// FP64 tensor-core (DMMA, mma.sync m8n8k4 f64) batched GEMM.  A warp owns a
-// (8 TI) x (8 TJ) block of C held as TI*TJ 8x8 accumulator fragments; the CTA is a
-// WM x WN grid of warps, one CTA tile of one batch entry per block.  A and B stream
-// through a GST-stage ring of shared-memory buffers, GK deep along K, filled with
-// cp.async (8-byte copies, zero-filled outside the matrix) so no registers stage the
-// loads and up to GST-1 chunks are in flight while one is multiplied.  Tiles are stored
-// k-major with a row stride of 4 (mod 16) doubles: the fragment loads of each half-warp
-// and the cp.async writes of four consecutive k by four columns hit distinct banks.
-// Fragment layout (PTX ISA, m8n8k4 .f64): a0 = A[lane/4][lane%4], b0 = B[lane%4][lane/4],
-// c0/c1 = C[lane/4][2 (lane%4) + 0/1].
+// FP64 tensor-core (DMMA) batched GEMM.  A warp owns a (16 TI) x (8 TJ) block of C held as
+// TI TJ accumulators of mma.sync m16n8k8 f64; the CTA is a WM x WN grid of warps, one CTA tile of
+// one batch entry per block.  A and B stream through a GST-stage ring of shared-memory buffers,
+// GK deep along K, filled with cp.async (zero-filled outside the matrix) so no registers stage
+// the loads and up to GST-1 chunks are in flight while one is multiplied.  A is stored k-major
+// with a row stride of 4 (mod 16) doubles, B column by column with a stride of GK + 4: the
+// fragment loads of each half-warp hit distinct banks.  Element blocks of odd order leave only
+// 8-byte alignment, so the copies move one entry each; where every address is a multiple of 16
+// bytes (VEC) they move two.
+// Fragments (PTX ISA, m16n8k8 .f64; g = lane / 4, t = lane % 4): a0..a3 = A[g, t], A[g + 8, t],
+// A[g, t + 4], A[g + 8, t + 4]; b0, b1 = B[t, g], B[t + 4, g]; c0..c3 = C[g, 2t], C[g, 2t + 1],
+// C[g + 8, 2t], C[g + 8, 2t + 1].
+// Measured (B200; before: m8n8k4, 256 threads, 128 x 64 to 160 x 64 tiles, two CTAs per SM): 1000
+// products of 480 x 480 x 320 6.39 -> 5.57 ms (26.5 TFLOP/s of 37 that either mma shape reaches from
+// registers), of 320 x 480 x 320 3.89 -> 3.12 ms; 1331 of 125 x 125 x 375 724 -> 716 us.  ncu: the
+// tensor pipe is active 65 to 70% of the cycles, waits for copies and fixed latencies take the rest.
 // ----------------------------------------------------------------------------------
-constexpr int GK = 16, GST = 3;
+constexpr int GK = 16, GST = 3, GSB = GK + 4;
 
 __host__ __device__ constexpr int dmma_stride(int w) { return (w + 15) / 16 * 16 + 4; }
 
 template <int TI, int TJ, int WM, int WN>
 constexpr size_t dmma_smem() {
-  return sizeof(double) * (size_t)GST * GK * (dmma_stride(8 * TI * WM) + dmma_stride(8 * TJ * WN));
+  return sizeof(double) * (size_t)GST * (GK * dmma_stride(16 * TI * WM) + GSB * 8 * TJ * WN);
 }
 
-__device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
-               : "+d"(c0), "+d"(c1)
-               : "d"(a), "d"(b));
+__device__ __forceinline__ void dmma(double (&c)[4], const double (&a)[4], const double (&b)[2]) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, "
+      "%3};\n"
+      : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+      : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
 }
 
-// 8-byte asynchronous copy global -> shared; src_bytes = 0 writes zeros and reads nothing
-__device__ __forceinline__ void cp_async8(double* dst, const double* src, int src_bytes) {
+// asynchronous copy global -> shared of W doubles; the bytes past src_bytes are written as zeros
+template <int W>
+__device__ __forceinline__ void cp_async(double* dst, const double* src, int src_bytes) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src), "r"(src_bytes));
+  if constexpr (W == 1)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src), "r"(src_bytes));
+  else
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(src_bytes));
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
 
-template <int TI, int TJ, int WM, int WN>
-__global__ void __launch_bounds__(32 * WM * WN, 2) dmma_gemm_kernel(GemmBatch g) {
-  constexpr int BM = 8 * TI * WM, BN = 8 * TJ * WN, NT = 32 * WM * WN;
-  constexpr int SA = dmma_stride(BM), SB = dmma_stride(BN);
-  constexpr int LA = (BM * GK + NT - 1) / NT, LB = (BN * GK + NT - 1) / NT;
+template <int TI, int TJ, int WM, int WN, int MB, bool VEC>
+__global__ void __launch_bounds__(32 * WM * WN, MB) dmma_gemm_kernel(GemmBatch g) {
+  constexpr int BM = 16 * TI * WM, BN = 8 * TJ * WN, NT = 32 * WM * WN, W = VEC ? 2 : 1;
+  constexpr int SA = dmma_stride(BM);
+  constexpr int RA = BM / W, KB = GK / W;  // copies per column of A, per column of B
+  constexpr int LA = (RA * GK + NT - 1) / NT, LB = (KB * BN + NT - 1) / NT;
   extern __shared__ __align__(16) double dsm[];
   double* As = dsm;                    // [GST][GK][SA]
-  double* Bs = dsm + GST * GK * SA;    // [GST][GK][SB]
+  double* Bs = dsm + GST * GK * SA;    // [GST][BN][GSB]
   const int tilesM = (g.M + BM - 1) / BM;
   const int tm = blockIdx.x % tilesM, tn = blockIdx.x / tilesM;
   const long long b1 = blockIdx.y, b2 = blockIdx.z;
@@ -143,37 +156,38 @@ __global__ void __launch_bounds__(32 * WM * WN, 2) dmma_gemm_kernel(GemmBatch g)
   const int wm = warp % WM, wn = warp / WM;
   const int r0 = tm * BM, c0 = tn * BN;
   const int gq = lane >> 2, tq = lane & 3;
-  double acc[TI][TJ][2];
+  double acc[TI][TJ][4];
 #pragma unroll
   for (int i = 0; i < TI; ++i)
 #pragma unroll
-    for (int j = 0; j < TJ; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+    for (int j = 0; j < TJ; ++j)
+#pragma unroll
+      for (int h = 0; h < 4; ++h) acc[i][j][h] = 0.0;
   const int nk = (g.K + GK - 1) / GK;
-  // stage s <- K chunk kc.  A: consecutive threads take consecutive rows (contiguous in
-  // global and in shared memory).  B: groups of four threads take four consecutive k of
-  // one column (one 32-byte sector), the next group the next column.
+  // stage s <- K chunk kc.  Consecutive threads take consecutive rows of a column of A, and
+  // consecutive k of a column of B (KB threads per column).
   auto load = [&](int s, int kc) {
     const int k0 = kc * GK;
     double* as = As + s * GK * SA;
-    double* bs = Bs + s * GK * SB;
+    double* bs = Bs + s * BN * GSB;
 #pragma unroll
     for (int q = 0; q < LA; ++q) {
       const int t = tid + NT * q;
-      const int r = t % BM, k = t / BM;
-      if (k < GK) {
+      const int r = t % RA * W, k = t / RA;
+      if (RA * GK % NT == 0 || k < GK) {
         const int gr = r0 + r, gk = k0 + k;
-        const bool in = gr < g.M && gk < g.K;
-        cp_async8(as + k * SA + r, in ? A + gr + g.lda * gk : A, in ? 8 : 0);
+        const int nb = gk < g.K ? 8 * min(W, max(0, g.M - gr)) : 0;
+        cp_async<W>(as + k * SA + r, nb ? A + gr + g.lda * gk : A, nb);
       }
     }
 #pragma unroll
     for (int q = 0; q < LB; ++q) {
       const int t = tid + NT * q;
-      const int rest = t >> 2, c = rest % BN, k = (t & 3) + 4 * (rest / BN);
-      if (k < GK) {
+      const int k = t % KB * W, c = t / KB;
+      if (KB * BN % NT == 0 || c < BN) {
         const int gk = k0 + k, gc = c0 + c;
-        const bool in = gk < g.K && gc < g.N;
-        cp_async8(bs + k * SB + c, in ? B + gk + g.ldb * gc : B, in ? 8 : 0);
+        const int nb = gc < g.N ? 8 * min(W, max(0, g.K - gk)) : 0;
+        cp_async<W>(bs + c * GSB + k, nb ? B + gk + g.ldb * gc : B, nb);
       }
     }
   };
@@ -182,54 +196,73 @@ __global__ void __launch_bounds__(32 * WM * WN, 2) dmma_gemm_kernel(GemmBatch g)
     if (s < nk) load(s, s);
     cp_async_commit();
   }
-  const int wr = wm * 8 * TI, wc = wn * 8 * TJ;
+  const int wr = wm * 16 * TI, wc = wn * 8 * TJ;
   for (int kc = 0; kc < nk; ++kc) {
     cp_async_wait<GST - 2>();
     __syncthreads();  // chunk kc visible to all; the buffer of chunk kc-1 is free
     if (kc + GST - 1 < nk) load((kc + GST - 1) % GST, kc + GST - 1);
     cp_async_commit();
-    const double* as = As + (kc % GST) * GK * SA;
-    const double* bs = Bs + (kc % GST) * GK * SB;
+    const double* as = As + (kc % GST) * GK * SA + tq * SA + wr + gq;
+    const double* bs = Bs + (kc % GST) * BN * GSB + (wc + gq) * GSB + tq;
 #pragma unroll
-    for (int k4 = 0; k4 < GK; k4 += 4) {
-      double af[TI], bf[TJ];
+    for (int k8 = 0; k8 < GK; k8 += 8) {
+      double af[TI][4], bf[TJ][2];
 #pragma unroll
-      for (int i = 0; i < TI; ++i) af[i] = as[(k4 + tq) * SA + wr + 8 * i + gq];
+      for (int i = 0; i < TI; ++i) {
+        af[i][0] = as[k8 * SA + 16 * i];
+        af[i][1] = as[k8 * SA + 16 * i + 8];
+        af[i][2] = as[(k8 + 4) * SA + 16 * i];
+        af[i][3] = as[(k8 + 4) * SA + 16 * i + 8];
+      }
 #pragma unroll
-      for (int j = 0; j < TJ; ++j) bf[j] = bs[(k4 + tq) * SB + wc + 8 * j + gq];
+      for (int j = 0; j < TJ; ++j) {
+        bf[j][0] = bs[8 * j * GSB + k8];
+        bf[j][1] = bs[8 * j * GSB + k8 + 4];
+      }
 #pragma unroll
-      for (int i = 0; i < TI; ++i)
+      for (int j = 0; j < TJ; ++j)
 #pragma unroll
-        for (int j = 0; j < TJ; ++j) dmma(acc[i][j][0], acc[i][j][1], af[i], bf[j]);
+        for (int i = 0; i < TI; ++i) dmma(acc[i][j], af[i], bf[j]);
     }
   }
   cp_async_wait<0>();
 #pragma unroll
-  for (int i = 0; i < TI; ++i) {
-    const int gr = r0 + wr + 8 * i + gq;
-    if (gr >= g.M) continue;
+  for (int i = 0; i < TI; ++i)
 #pragma unroll
-    for (int j = 0; j < TJ; ++j)
+    for (int h = 0; h < 2; ++h) {
+      const int gr = r0 + wr + 16 * i + 8 * h + gq;
+      if (gr >= g.M) continue;
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int gc = c0 + wc + 8 * j + 2 * tq + h;
-        if (gc >= g.N) continue;
-        double* p = C + gr + g.ldc * gc;
-        const double v = g.alpha * acc[i][j][h];
-        *p = (g.beta == 0.0) ? v : v + g.beta * (*p);
-      }
-  }
+      for (int j = 0; j < TJ; ++j)
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+          const int gc = c0 + wc + 8 * j + 2 * tq + x;
+          if (gc >= g.N) continue;
+          double* p = C + gr + g.ldc * gc;
+          const double v = g.alpha * acc[i][j][2 * h + x];
+          *p = (g.beta == 0.0) ? v : v + g.beta * (*p);
+        }
+    }
 }
 
-template <int TI, int TJ, int WM, int WN>
+template <int TI, int TJ, int WM, int WN, int MB>
 int launch_dmma(const GemmBatch& g, cudaStream_t st) {
-  constexpr int BM = 8 * TI * WM, BN = 8 * TJ * WN;
+  constexpr int BM = 16 * TI * WM, BN = 8 * TJ * WN;
   constexpr size_t smem = dmma_smem<TI, TJ, WM, WN>();
-  static_assert(smem <= 227 * 1024, "GEMM tile exceeds shared memory");
-  auto kern = dmma_gemm_kernel<TI, TJ, WM, WN>;
-  EXA_TRY(exa_allow_smem((const void*)kern, smem));
+  static_assert(MB * smem <= 227 * 1024, "GEMM tiles exceed shared memory");
+  // pairs of entries where every copy then starts on a 16-byte boundary
+  const bool vec = ((reinterpret_cast<uintptr_t>(g.A) | reinterpret_cast<uintptr_t>(g.B)) & 15) == 0 &&
+                   ((g.lda | g.sA | g.sA2 | g.ldb | g.sB | g.sB2) & 1) == 0;
   dim3 grid((unsigned)(exa_ceil_div(g.M, BM) * exa_ceil_div(g.N, BN)), (unsigned)g.batch, (unsigned)g.batch2);
-  kern<<<grid, 32 * WM * WN, smem, st>>>(g);
+  if (vec) {
+    auto kern = dmma_gemm_kernel<TI, TJ, WM, WN, MB, true>;
+    EXA_TRY(exa_allow_smem((const void*)kern, smem));
+    kern<<<grid, 32 * WM * WN, smem, st>>>(g);
+  } else {
+    auto kern = dmma_gemm_kernel<TI, TJ, WM, WN, MB, false>;
+    EXA_TRY(exa_allow_smem((const void*)kern, smem));
+    kern<<<grid, 32 * WM * WN, smem, st>>>(g);
+  }
   EXA_LAUNCH_CHECK();
   return EXA_OK;
 }
@@ -238,27 +271,28 @@ long long tiles_cost(int M, int N, int bm, int bn) {
   return (long long)((M + bm - 1) / bm) * bm * ((N + bn - 1) / bn) * bn;
 }
 
-// CTA tiles sized to the element blocks: 128 x 64, 128 x 80, 160 x 32 and 160 x 64 cover
-// 125 -> 128 and 150 -> 160 with little padding; 64 x 128 and 64 x 64 fit the chunk-wide
-// products with 64 rows (Gauss points or nodes of a p = 3 hexahedron) and long rows of columns
+// CTA tiles sized to the element blocks: multiples of 64 and 80 cover 125 -> 128, 150 -> 160 and
+// the 160, 320 and 480 of the large blocks with little padding; three CTAs of 4 or 5 warps share
+// an SM, so one's barrier or epilogue overlaps the others' products.  128 x 64 and 64 x 128 halve
+// the reads of one operand.
 constexpr int kTiles = 6;
-constexpr int kTile[kTiles][2] = {{128, 64}, {128, 80}, {160, 32}, {160, 64}, {64, 128}, {64, 64}};
+constexpr int kTile[kTiles][2] = {{64, 64}, {64, 80}, {80, 64}, {80, 80}, {128, 64}, {64, 128}};
 
 int launch_tile(int t, const GemmBatch& g, cudaStream_t st) {
   switch (t) {
-    case 0: return launch_dmma<4, 4, 4, 2>(g, st);
-    case 1: return launch_dmma<4, 5, 4, 2>(g, st);
-    case 2: return launch_dmma<5, 2, 4, 2>(g, st);
-    case 3: return launch_dmma<5, 4, 4, 2>(g, st);
-    case 4: return launch_dmma<2, 8, 4, 2>(g, st);
-    default: return launch_dmma<2, 4, 4, 2>(g, st);
+    case 0: return launch_dmma<2, 4, 2, 2, 3>(g, st);
+    case 1: return launch_dmma<2, 5, 2, 2, 3>(g, st);
+    case 2: return launch_dmma<1, 8, 5, 1, 3>(g, st);
+    case 3: return launch_dmma<1, 10, 5, 1, 3>(g, st);
+    case 4: return launch_dmma<2, 4, 4, 2, 2>(g, st);
+    default: return launch_dmma<2, 4, 2, 4, 2>(g, st);
   }
 }
 
 std::mutex g_tune_mu;
 std::map<std::array<int, 4>, int> g_tune;  // (device, M, N, K) -> measured fastest tile
 
-// the measured tile of this shape, else the least padded of 128 x 64, 128 x 80 and 160 x 32
+// the measured tile of this shape, else the least padded, the largest of those that tie
 int gemm_tile(int M, int N, int K) {
   int dev = 0;
   if (cudaGetDevice(&dev) == cudaSuccess) {
@@ -268,9 +302,12 @@ int gemm_tile(int M, int N, int K) {
   }
   int best = 0;
   long long bc = -1;
-  for (int i = 0; i < 3; ++i) {
+  for (int i = 0; i < kTiles; ++i) {
     const long long c = tiles_cost(M, N, kTile[i][0], kTile[i][1]);
-    if (bc < 0 || c < bc) { bc = c; best = i; }
+    if (bc < 0 || c < bc || (c == bc && kTile[i][0] * kTile[i][1] > kTile[best][0] * kTile[best][1])) {
+      bc = c;
+      best = i;
+    }
   }
   return best;
 }
@@ -300,7 +337,7 @@ int exa_gemm(const GemmBatch& g, cudaStream_t st) {
     EXA_LAUNCH_CHECK();
     return EXA_OK;
   }
-  if (g.M <= 40 && g.N <= 40) return launch_dmma<2, 2, 2, 2>(g, st);
+  if (g.M <= 40 && g.N <= 40) return launch_dmma<1, 2, 2, 2, 4>(g, st);
   return launch_tile(gemm_tile(g.M, g.N, g.K), g, st);
 }
 
