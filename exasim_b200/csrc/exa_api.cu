@@ -368,6 +368,7 @@ int exa_ctx_init(ExaCtx& c, const double* app, long long napp, const double* mas
   EXA_TRY(dev_alloc(c, &c.elemg, ne * P.elemg_stride()));
   EXA_TRY(dev_alloc(c, &c.faceg, ne * P.nfe * P.faceg_stride()));
   EXA_TRY(exa_k_geometry(P, c.shapegt, c.shapfgt, c.perm, c.xdg, c.elemg, c.faceg, c.st));
+  find_tensor(c.tensor, M, P, c.elemtype);
   if (c.scheme == 0) {
     // LDG: both sides' face-node table, the face nodal basis for the boundary's Ubou, and
     // the residual buffers of the finite-difference Jacobian
@@ -390,7 +391,6 @@ int exa_ctx_init(ExaCtx& c, const double* app, long long napp, const double* mas
     EXA_TRY(dev_alloc(c, &c.ldg_fcon, 2 * (size_t)P.npf * P.nf));
     EXA_TRY(exa_k_ldg_fcon(P, c.f2e, c.perm, c.elemcon, c.ldg_fcon, c.st));
     // tensor-product elements: the tables of the element kernel (every node on at most nd faces)
-    find_tensor(c.tensor, M, P, c.elemtype);
     if (c.tensor.n1 > 0 && c.ldg_split && (long long)P.npf * P.ncu * P.nf < (1LL << 31)) {
       std::vector<int> ns((size_t)P.nd * P.npe, -1);
       bool ok = true;
@@ -518,7 +518,7 @@ int exa_ctx_init(ExaCtx& c, const double* app, long long napp, const double* mas
   EXA_TRY(dev_alloc(c, &c.wUG, nb * P.nge * P.nc));
   EXA_TRY(dev_alloc(c, &c.wSG, nb * P.nge * P.ncu));
   EXA_TRY(dev_alloc(c, &c.wRG, nb * P.nge * (P.nd + 1) * P.ncu));
-  if (hdg) {
+  if (hdg && !exa_tensor_blocks(P, c.tensor)) {
     // T factors of the FP64 volume products: at most 512 MB, the chunk taken in parts
     const size_t per = (size_t)P.npe * P.nge * P.ncu * P.nc;
     c.wT_elems = (int)std::max<size_t>(1, std::min<size_t>(nb, (512u << 20) / (8 * per)));
@@ -545,7 +545,7 @@ int exa_ctx_init(ExaCtx& c, const double* app, long long napp, const double* mas
     }
     EXA_TRY(exa_gemm_tune((int)n, (int)m, (int)n, nbt, c.st));
     EXA_TRY(exa_gemm_tune((int)m, (int)m, (int)n, nbt, c.st));
-    EXA_TRY(exa_gemm_tune(P.npe, P.npe, P.nge, nbt, c.st));  // the FP64 volume products
+    if (c.wT) EXA_TRY(exa_gemm_tune(P.npe, P.npe, P.nge, nbt, c.st));  // the FP64 volume products
     // and the element inverse (FP64 D of the plain form)
     EXA_TRY(exa_inverse_tune((int)n, (int)std::min<size_t>(nb, 4096), 1, c.st));
   }

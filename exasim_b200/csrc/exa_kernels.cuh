@@ -55,6 +55,10 @@ struct ExaTensor {
   int n1 = 0;
   double S[EXA_TP_MAX * EXA_TP_MAX], D[EXA_TP_MAX * EXA_TP_MAX], w[EXA_TP_MAX];  // S[g + n1 a]
 };
+// whether the volume blocks of such elements go by sum factorization (exa_vol_tp.cuh)
+inline bool exa_tensor_blocks(const ExaDims& P, const ExaTensor& T) {
+  return (P.nd == 2 || P.nd == 3) && T.n1 >= 3 && T.n1 <= 5;
+}
 struct ExaSweepDev {
   int levels = 0;
   int *lev = nullptr, *row = nullptr, *ptr = nullptr, *blk = nullptr;

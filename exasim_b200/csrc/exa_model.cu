@@ -8,6 +8,7 @@
 #include "exa_assembly.cuh"
 #include "exa_ldg.cuh"
 #include "exa_ldg_tp.cuh"
+#include "exa_vol_tp.cuh"
 #include "exa_solver.cuh"
 #include "exa_umma.cuh"
 #include EXA_MODEL_HEADER
@@ -388,16 +389,22 @@ int exa_model_assemble(ExaCtx& c, bool jacobian) {
         vol_points_kernel<ExaModel, true><<<nb, tpb_v, vs, c.st>>>(A, Ruc, c.wRg);
         EXA_LAUNCH_CHECK();
         if (c.wRG) EXA_TRY(volume_residual_gemm(c, Ruc, nb));
-        if (c.precision == 1 && c.Sp.hi) {
-          // B straight into its packed FP32 form (the face kernel adds its terms there too).
-          // The volume kernel assigns every entry of B, so only the layout's padding needs
-          // zeros, and nothing writes there after the zeroing at allocation.
-          UPacked bp{};
-          if (nqn > 0 && P.ncq > 0) {
-            bp = c.wBp;
-            A.Bp = c.wBp;
-          }
+        // B straight into its packed FP32 form where the mixed form's q elimination takes it (the
+        // face kernel adds its terms there too).  The volume kernel assigns every entry of B, so
+        // only the layout's padding needs zeros, and nothing writes there after the zeroing at
+        // allocation.
+        const bool packed = c.precision == 1 && c.Sp.hi;
+        UPacked bp{};
+        if (packed && nqn > 0 && P.ncq > 0) {
+          bp = c.wBp;
+          A.Bp = c.wBp;
+        }
+        int rc = EXA_OK;
+        if (packed) {
           EXA_TRY(exa_k_vol_mat_tc(P, c.shapegw32, c.Sp, c.wRg, c.wD, c.wB, bp, nb, c.d_uflag, c.st));
+        } else if (exa_tensor_blocks(P, c.tensor) &&
+                   launch_vol_blocks_tp(P, c.tensor, c.wRg, c.wD, c.wB, nb, c.st, &rc)) {
+          EXA_TRY(rc);
         } else if (c.wT) {
           EXA_TRY(volume_blocks_gemm(c, nb));
         } else {
