@@ -170,6 +170,11 @@ int ldg_matvec(ExaCtx& c, const double* v, double* w) {
 int exa_drv_matvec(ExaCtx& c, const double* v, double* w) {
   ExaProfScope ps(c, EXA_PH_MATVEC);
   if (c.scheme == 0) return ldg_matvec(c, v, w);
+  if (v != w && exa_face_op_fits(c.P, c.precision == 1 ? 4 : 8)) {
+    if (c.precision == 1)
+      return exa_k_face_op<float>(c.P, c.f2e, c.elemcon, c.H32, nullptr, v, w, nullptr, c.st);
+    return exa_k_face_op<double>(c.P, c.f2e, c.elemcon, c.H, nullptr, v, w, nullptr, c.st);
+  }
   if (c.precision == 1)
     EXA_TRY(exa_k_elem_matvec(c.P, c.elemcon, c.H32, v, c.we, c.st, c.d_uflag));
   else
@@ -226,8 +231,15 @@ extern "C" int exa_poly_ritz(const double* H, int m, double* sr, double* si);
 
 namespace {
 
-// out = P A x (x may be out): the matvec into c.w, then the preconditioner
+// out = P A x (x may be out): the matvec into c.w, then the preconditioner; small block-Jacobi
+// systems in one launch
 int pa(ExaCtx& c, const double* x, double* out) {
+  if (c.scheme != 0 && c.preconditioner == 0 && x != out && exa_face_op_fits(c.P, c.precision == 1 ? 4 : 8)) {
+    ExaProfScope ps(c, EXA_PH_MATVEC);
+    if (c.precision == 1)
+      return exa_k_face_op<float>(c.P, c.f2e, c.elemcon, c.H32, c.Pc32, x, nullptr, out, c.st);
+    return exa_k_face_op<double>(c.P, c.f2e, c.elemcon, c.H, c.Pc, x, nullptr, out, c.st);
+  }
   EXA_TRY(exa_drv_matvec(c, x, c.w));
   return exa_drv_precond(c, c.w, out);
 }
@@ -313,8 +325,7 @@ int arnoldi_ops(ExaCtx& c, int i, const double* d_nrmb, double* d_relerr, double
   double* vi = c.V + (long long)i * N;
   double* vn = c.V + (long long)(i + 1) * N;
   double* hcol = c.hess + (long long)n1 * i;
-  EXA_TRY(exa_drv_matvec(c, vi, c.w));
-  EXA_TRY(exa_drv_precond(c, c.w, vn));
+  EXA_TRY(pa(c, vi, vn));
   EXA_TRY(apply_poly(c, vn));
   {
     ExaProfScope ps_ortho(c, EXA_PH_ORTHO);

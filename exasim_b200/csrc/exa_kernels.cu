@@ -242,6 +242,80 @@ __global__ void bj_apply_kernel(ExaDims P, const T* BE, const double* x, double*
   }
 }
 
+// The condensed matvec and the block-Jacobi apply face by face: w_f = sum over the face's elements
+// of their block's rows on f times the gathered v, then (y given) y_f = BE_f w_f.  One launch in
+// place of the element products, their scatter and the apply, without the element vectors between.
+// For small systems, where launches and latency are the time (B200: A v on 144 faces of 3 rows with
+// the apply, two calls, 26.9 -> 24.3 us; 245 GMRES steps on 1200 faces of 4 rows 8.3 -> 5.8 ms);
+// wpf warps share a face's columns.
+// Sums: each lane its columns in order, lanes by a fixed shuffle tree, warps and sides in order.
+constexpr int FO_ROWS = 32;
+constexpr double FACE_OP_BYTES = 32e6;
+template <typename T>
+__global__ void __launch_bounds__(256) face_op_kernel(ExaDims P, const int* f2e, const int* elemcon, const T* H,
+                                                      const T* BE, const double* v, double* w, double* y, int wpf) {
+  __shared__ double part[8][FO_ROWS];
+  __shared__ double wf[8][FO_ROWS];
+  const int ncu = P.ncu, npf = P.npf, ncf = ncu * npf, m = P.m, ndf = P.ndf;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, slot = warp / wpf, sub = warp - slot * wpf;
+  const int f = blockIdx.x * (8 / wpf) + slot;
+  const bool on = f < P.nf;
+  int rp = 4;  // lanes per column: a power of two that holds the rows
+  while (rp < ncf) rp *= 2;
+  const int r = lane & (rp - 1), g = 32 / rp, c0 = lane / rp + g * sub, step = g * wpf;
+  double s = 0.0;
+  if (on && r < ncf) {
+    const int e1 = f2e[4 * f], l1 = f2e[4 * f + 1], e2 = f2e[4 * f + 2], l2 = f2e[4 * f + 3];
+    for (int side = 0; side < 2; ++side) {
+      if (side == 1 && (f >= P.nf0 || e2 < 0)) break;
+      const int e = side ? e2 : e1, l = side ? l2 : l1;
+      const int* con = elemcon + (long long)ndf * e;
+      const int row = side ? r % ncu + ncu * (con[r / ncu + npf * l] - npf * f) + ncf * l : r + ncf * l;
+      const T* Hr = H + (long long)e * m * m + row;
+      double t = 0.0;
+      for (int c = c0; c < m; c += 8 * step) {
+        T a[8];
+        double x[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const int cc = c + u * step;
+          a[u] = cc < m ? Hr[(long long)m * cc] : T(0);
+          x[u] = cc < m ? v[ncu == 1 ? con[cc] : cc % ncu + ncu * con[cc / ncu]] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) t = fma((double)a[u], x[u], t);
+      }
+      s += t;
+    }
+  }
+  for (int off = rp; off < 32; off *= 2) s += __shfl_xor_sync(0xffffffffu, s, off);
+  if (lane < ncf) part[warp][lane] = s;
+  __syncthreads();
+  if (sub != 0) return;
+  if (on && lane < ncf) {
+    double t = 0.0;
+    for (int q = 0; q < wpf; ++q) t += part[warp + q][lane];
+    wf[slot][lane] = t;
+    if (w) w[(long long)ncf * f + lane] = t;
+  }
+  if (!y || !on) return;
+  __syncwarp();
+  double t = 0.0;
+  if (r < ncf) {
+    const T* A = BE + (long long)ncf * ncf * f + r;
+    for (int c = lane / rp; c < ncf; c += 8 * g) {
+      T a[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) a[u] = c + u * g < ncf ? A[ncf * (c + u * g)] : T(0);
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (c + u * g < ncf) t = fma((double)a[u], wf[slot][c + u * g], t);
+    }
+  }
+  for (int off = rp; off < 32; off *= 2) t += __shfl_xor_sync(0xffffffffu, t, off);
+  if (lane < ncf) y[(long long)ncf * f + lane] = t;
+}
+
 // y_e = alpha A_e x_e + beta y0_e for a batch of column-major M x K blocks A_e (leading
 // dimension M, batch stride sA; y0 may alias y).  x_e is read at x + e sx, or, with elemcon,
 // gathered from a trace vector: x_e[k] = x[k % ncu + ncu elemcon[k / ncu + ndf e]].  One
@@ -955,6 +1029,22 @@ int exa_k_elem_matvec(const ExaDims& P, const int* elemcon, const T* A, const do
                          P.m, st, flag);
 }
 
+// Face by face where the blocks lie in L2 (both elements of a face read rows of theirs, in pieces
+// of a column) and a face's rows fit a warp's lanes; larger systems read whole blocks at the HBM
+// rate through exa_k_elem_matvec.
+bool exa_face_op_fits(const ExaDims& P, int entry_bytes) {
+  return P.ncu * P.npf <= FO_ROWS && (double)entry_bytes * P.m * P.m * P.ne <= FACE_OP_BYTES;
+}
+
+template <typename T>
+int exa_k_face_op(const ExaDims& P, const int* f2e, const int* elemcon, const T* H, const T* BE, const double* v,
+                  double* w, double* y, cudaStream_t st) {
+  const int wpf = P.m <= 32 ? 1 : (P.m <= 64 ? 2 : (P.m <= 96 ? 4 : 8));
+  face_op_kernel<T><<<exa_ceil_div(P.nf, 8 / wpf), 256, 0, st>>>(P, f2e, elemcon, H, BE, v, w, y, wpf);
+  EXA_LAUNCH_CHECK();
+  return EXA_OK;
+}
+
 template <typename T>
 int exa_k_bj_build(const ExaDims& P, const int* f2e, const int* elemcon, const T* H, T* BE, cudaStream_t st) {
   const long long ncf = (long long)P.ncu * P.npf;
@@ -1072,6 +1162,8 @@ int exa_k_to_f32(const double* x, float* y, long long n, cudaStream_t st) {
                                     int*);                                                                     \
   template int exa_k_bj_build<T>(const ExaDims&, const int*, const int*, const T*, T*, cudaStream_t);           \
   template int exa_k_eas_build<T>(const ExaDims&, const int*, const int*, const T*, T*, cudaStream_t);          \
+  template int exa_k_face_op<T>(const ExaDims&, const int*, const int*, const T*, const T*, const double*,        \
+                                double*, double*, cudaStream_t);                                               \
   template int exa_k_bj_apply<T>(const ExaDims&, const T*, const double*, double*, cudaStream_t);              \
   template int exa_k_dudg<T>(const ExaDims&, const int*, const T*, const double*, const double*, double*, cudaStream_t, \
                              int*);

@@ -23,6 +23,12 @@ int exa_k_scatter(const ExaDims& P, const int* f2e, const int* elemcon, const do
 template <typename T>
 int exa_k_elem_matvec(const ExaDims& P, const int* elemcon, const T* A, const double* v, double* we,
                       cudaStream_t st, int* flag = nullptr);
+// w = A v and, with y, y = block-Jacobi apply of w, in one launch (BE and w may be null); for the
+// systems exa_face_op_fits takes.  v must not be w or y.
+bool exa_face_op_fits(const ExaDims& P, int entry_bytes);
+template <typename T>
+int exa_k_face_op(const ExaDims& P, const int* f2e, const int* elemcon, const T* H, const T* BE, const double* v,
+                  double* w, double* y, cudaStream_t st);
 template <typename T>
 int exa_k_bj_build(const ExaDims& P, const int* f2e, const int* elemcon, const T* H, T* BE, cudaStream_t st);
 template <typename T>
