@@ -636,8 +636,8 @@ __device__ __forceinline__ void warp_argmax(T best, int bi, int n, T& mbest, int
   }
 }
 
-template <typename T, int NW, int CW, int RL>
-__global__ void __launch_bounds__(32 * NW, sizeof(T) == 4 ? 2 : 1)
+template <typename T, int NW, int CW, int RL, int MB>
+__global__ void __launch_bounds__(32 * NW, MB)
     inverse_wcol_kernel(T* Aall, int n, long long stride, int* flag) {
   __shared__ T colb[2][32 * RL];
   __shared__ int sp[2];
@@ -781,18 +781,23 @@ __global__ void __launch_bounds__(32 * NW, sizeof(T) == 4 ? 2 : 1)
     }
 }
 
-// The column-by-warp shapes: warps x columns per warp x rows per lane.  Variants 0-1 hold up
-// to 128 rows and columns, 2-3 up to 64.  exa_inverse_tune times them per order and type.
+// The column-by-warp shapes: warps x columns per warp x rows per lane, by the largest order they
+// hold (three sizes, so that a block pads little and as many CTAs as possible share an SM and hide
+// one another's pivot chains), two each.  exa_inverse_tune times both per order and type.  Measured
+// (B200, 3000 blocks of order 80; before: the shapes for 128): FP64 1.55 -> 0.73 ms, FP32 0.71 -> 0.43 ms.
 constexpr int kInvVariants = 4;
-__host__ __device__ constexpr int inv_variant_nmax(int v) { return v < 2 ? 128 : 64; }
+inline int inv_shape(int n, int v) { return (n <= 64 ? 4 : (n <= 96 ? 2 : 0)) + (v & 1); }
 
 template <typename T>
 int launch_wcol(int v, T* A, int n, long long stride, int batch, int* d_flag, cudaStream_t st) {
-  switch (v) {
-    case 0: inverse_wcol_kernel<T, 8, 16, 4><<<batch, 256, 0, st>>>(A, n, stride, d_flag); break;
-    case 1: inverse_wcol_kernel<T, 16, 8, 4><<<batch, 512, 0, st>>>(A, n, stride, d_flag); break;
-    case 2: inverse_wcol_kernel<T, 4, 16, 2><<<batch, 128, 0, st>>>(A, n, stride, d_flag); break;
-    default: inverse_wcol_kernel<T, 8, 8, 2><<<batch, 256, 0, st>>>(A, n, stride, d_flag); break;
+  constexpr bool F = sizeof(T) == 4;
+  switch (inv_shape(n, v)) {
+    case 0: inverse_wcol_kernel<T, 8, 16, 4, F ? 2 : 1><<<batch, 256, 0, st>>>(A, n, stride, d_flag); break;
+    case 1: inverse_wcol_kernel<T, 16, 8, 4, F ? 2 : 1><<<batch, 512, 0, st>>>(A, n, stride, d_flag); break;
+    case 2: inverse_wcol_kernel<T, 6, 16, 3, F ? 3 : 2><<<batch, 192, 0, st>>>(A, n, stride, d_flag); break;
+    case 3: inverse_wcol_kernel<T, 12, 8, 3, F ? 2 : 1><<<batch, 384, 0, st>>>(A, n, stride, d_flag); break;
+    case 4: inverse_wcol_kernel<T, 4, 16, 2, F ? 6 : 4><<<batch, 128, 0, st>>>(A, n, stride, d_flag); break;
+    default: inverse_wcol_kernel<T, 8, 8, 2, F ? 4 : 3><<<batch, 256, 0, st>>>(A, n, stride, d_flag); break;
   }
   EXA_LAUNCH_CHECK();
   return EXA_OK;
@@ -801,8 +806,8 @@ int launch_wcol(int v, T* A, int n, long long stride, int batch, int* d_flag, cu
 std::mutex g_inv_mu;
 std::map<std::array<int, 3>, int> g_inv_tune;  // (device, n, fp64) -> measured fastest variant
 
-// the measured variant for this order and type, else the default: FP32 8 warps x 16 columns
-// (4 warps up to 64), FP64 16 warps x 8 columns (8 x 8 up to 64)
+// the measured variant for this order and type (2, 3: the shapes for orders up to 64), else the
+// default: FP32 16 columns per warp, FP64 8
 int inv_variant(int n, bool fp64) {
   int dev = 0;
   if (cudaGetDevice(&dev) == cudaSuccess) {
@@ -810,7 +815,7 @@ int inv_variant(int n, bool fp64) {
     auto it = g_inv_tune.find({dev, n, fp64 ? 1 : 0});
     if (it != g_inv_tune.end()) return it->second;
   }
-  if (fp64) return n <= 64 ? 3 : 1;
+  if (fp64) return n <= 64 ? 3 : (n <= 96 ? 0 : 1);
   return n <= 64 ? 2 : 0;
 }
 
@@ -897,7 +902,7 @@ int inverse_tune(int n, int batch, cudaStream_t st) {
   int best = inv_variant(n, sizeof(T) == 8);
   float best_ms = -1.0f;
   for (int v = 0; v < kInvVariants && e == cudaSuccess; ++v) {
-    if (n > inv_variant_nmax(v)) continue;
+    if ((v >= 2) != (n <= 64)) continue;
     inv_tune_fill_kernel<T><<<1024, 256, 0, st>>>(buf, n, total);
     if (launch_wcol<T>(v, buf, n, (long long)n * n, nb, flag, st) != EXA_OK) break;  // warm
     e = cudaEventRecord(e0, st);
@@ -1030,10 +1035,15 @@ int subcopy(T* dst, long long ldd, long long sd, const T* src, long long lds, lo
   return EXA_OK;
 }
 
+// The diagonal blocks are inverted the same way down to INV_LEAF (order 320: leaves of 80, whose
+// register kernel keeps several CTAs on an SM; one CTA per SM held a 160 x 160 leaf), in the part of
+// the workspace that is not in use yet.  1000 blocks of order 320 13.0 -> 9.8 ms (B200).  sw: entries
+// between matrices in the workspace.
+constexpr int INV_LEAF = 96;
 template <typename T>
-int inverse_blocked(T* A, int n, long long stride, int batch, T* ws, int* d_flag, cudaStream_t st) {
+int inverse_blocked(T* A, int n, long long stride, int batch, T* ws, long long sw, int* d_flag, cudaStream_t st) {
+  if (n <= INV_LEAF) return inverse_dispatch<T>(A, n, stride, batch, d_flag, st);
   const int n1 = (n + 1) / 2, n2 = n - n1;
-  const long long sw = (long long)n * n;
   T* W0 = ws;                                  // n1 x n1: A11, then X
   T* W1 = W0 + (long long)n1 * n1;             // n1 x n2: X A12
   T* W2 = W1 + (long long)n1 * n2;             // n2 x n2: S, then Y
@@ -1043,11 +1053,11 @@ int inverse_blocked(T* A, int n, long long stride, int batch, T* ws, int* d_flag
   T* A12 = A + (long long)n * n1;
   T* A22 = A + n1 + (long long)n * n1;
   EXA_TRY(subcopy<T>(W0, n1, sw, A11, n, stride, n1, n1, batch, st));
-  EXA_TRY(inverse_dispatch<T>(W0, n1, sw, batch, d_flag, st));
+  EXA_TRY(inverse_blocked<T>(W0, n1, sw, batch, W1, sw, d_flag, st));
   EXA_TRY(bgemm<T>(n1, n2, n1, T(1), T(0), W0, n1, sw, A12, n, stride, W1, n1, sw, batch, st));
   EXA_TRY(bgemm<T>(n2, n2, n1, T(-1), T(1), A21, n, stride, W1, n1, sw, A22, n, stride, batch, st));
   EXA_TRY(subcopy<T>(W2, n2, sw, A22, n, stride, n2, n2, batch, st));
-  EXA_TRY(inverse_dispatch<T>(W2, n2, sw, batch, d_flag, st));
+  EXA_TRY(inverse_blocked<T>(W2, n2, sw, batch, W3, sw, d_flag, st));
   EXA_TRY(bgemm<T>(n2, n1, n1, T(1), T(0), A21, n, stride, W0, n1, sw, W3, n2, sw, batch, st));
   EXA_TRY(bgemm<T>(n1, n2, n2, T(-1), T(0), W1, n1, sw, W2, n2, sw, A12, n, stride, batch, st));
   EXA_TRY(subcopy<T>(A11, n, stride, W0, n1, sw, n1, n1, batch, st));
@@ -1068,7 +1078,7 @@ int inverse_ws(T* A, int n, long long stride, int batch, T* ws, int* d_flag, cud
     exa_set_error("dense inverse of order %d needs a workspace of n^2 entries per matrix", n);
     return EXA_ERR_ARG;
   }
-  return inverse_blocked<T>(A, n, stride, batch, ws, d_flag, st);
+  return inverse_blocked<T>(A, n, stride, batch, ws, (long long)n * n, d_flag, st);
 }
 }  // namespace
 
