@@ -29,6 +29,12 @@ def test_apply_matches_oracle(tmp_path, model, n, p, cgp):
     else:
         cases.convdiff3d_hex(d, n=n, porder=p, nsteps=1, preconditioner=2, cartgridpart=cgp)
     s, o = HDGSolver(d, model), HDGOracle(d, MODELS[model]())
+    if o.tdep:
+        o.sdg = 41.0 * o.udg[:, :o.ncu]
+        o.sdgg = np.einsum("gj,jce->gec", o.shapegt[:, :, 0], o.sdg)
+        o.time, o.dtfactor = 0.01, 40.0
+        s.set("sdg", o.sdg)
+        s.set_time(o.time, o.dtfactor)
     s.hdgGetQ()
     o.get_q(o.udg, o.uh)
     s.hdgAssembleLinearSystem()
