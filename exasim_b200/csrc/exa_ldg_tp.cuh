@@ -358,8 +358,9 @@ bool launch_ldg_tp(const LdgArgs& F, const AsmArgs& A, const LdgState& U, const 
     }();                                                                                                         \
     return true;                                                                                                 \
   }
-  // the pairs that a model of the package without q has; p = 2 to 4
-  EXA_LTP(3, 5, 3) EXA_LTP(3, 5, 4) EXA_LTP(3, 5, 5)
+  // the pairs that a model of the package without q has; p = 2 and 3 (contexts refuse element blocks
+  // above 320 x 320)
+  EXA_LTP(3, 5, 3) EXA_LTP(3, 5, 4)
 #undef EXA_LTP
   return false;
 }

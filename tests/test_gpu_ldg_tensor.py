@@ -16,8 +16,8 @@ from oracle.models import MODELS
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n,p,periodic", [(3, 1, True), (3, 2, True), (3, 3, True), (3, 4, True), (2, 2, False),
-                                          (3, 3, False), (1, 4, False)])
+@pytest.mark.parametrize("n,p,periodic", [(3, 1, True), (3, 2, True), (3, 3, True), (2, 2, False),
+                                          (3, 3, False), (1, 3, False)])
 def test_residual_and_product_match_oracle(tmp_path, n, p, periodic):
     import torch
     B.build(["euler3d"])
