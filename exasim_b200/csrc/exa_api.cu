@@ -369,6 +369,18 @@ int exa_ctx_init(ExaCtx& c, const double* app, long long napp, const double* mas
   EXA_TRY(dev_alloc(c, &c.faceg, ne * P.nfe * P.faceg_stride()));
   EXA_TRY(exa_k_geometry(P, c.shapegt, c.shapfgt, c.perm, c.xdg, c.elemg, c.faceg, c.st));
   find_tensor(c.tensor, M, P, c.elemtype);
+  if (c.tensor.n1 > 0) {
+    std::vector<int> ns((size_t)P.nd * P.npe, -1);
+    bool ok = true;
+    for (int t = 0; t < P.ndf && ok; ++t) {
+      int* q = &ns[(size_t)P.nd * perm[t]];
+      int k = 0;
+      while (k < P.nd && q[k] >= 0) ++k;
+      ok = k < P.nd;
+      if (ok) q[k] = t;
+    }
+    if (ok) EXA_TRY(dev_upload(c, &c.tp_nslot, ns.data(), ns.size()));
+  }
   if (c.scheme == 0) {
     // LDG: both sides' face-node table, the face nodal basis for the boundary's Ubou, and
     // the residual buffers of the finite-difference Jacobian
@@ -390,22 +402,9 @@ int exa_ctx_init(ExaCtx& c, const double* app, long long napp, const double* mas
     }
     EXA_TRY(dev_alloc(c, &c.ldg_fcon, 2 * (size_t)P.npf * P.nf));
     EXA_TRY(exa_k_ldg_fcon(P, c.f2e, c.perm, c.elemcon, c.ldg_fcon, c.st));
-    // tensor-product elements: the tables of the element kernel (every node on at most nd faces)
-    if (c.tensor.n1 > 0 && c.ldg_split && (long long)P.npf * P.ncu * P.nf < (1LL << 31)) {
-      std::vector<int> ns((size_t)P.nd * P.npe, -1);
-      bool ok = true;
-      for (int t = 0; t < P.ndf && ok; ++t) {
-        int* s = &ns[(size_t)P.nd * perm[t]];
-        int q = 0;
-        while (q < P.nd && s[q] >= 0) ++q;
-        ok = q < P.nd;
-        if (ok) s[q] = t;
-      }
-      if (ok) {
-        EXA_TRY(dev_upload(c, &c.ldg_nslot, ns.data(), ns.size()));
-        EXA_TRY(dev_alloc(c, &c.ldg_fslot, (size_t)P.ndf * P.ne));
-        EXA_TRY(exa_k_ldg_slots(P, c.f2e, c.elemcon, c.ldg_fslot, c.st));
-      }
+    if (c.tp_nslot && c.ldg_split && (long long)P.npf * P.ncu * P.nf < (1LL << 31)) {
+      EXA_TRY(dev_alloc(c, &c.ldg_fslot, (size_t)P.ndf * P.ne));
+      EXA_TRY(exa_k_ldg_slots(P, c.f2e, c.elemcon, c.ldg_fslot, c.st));
     }
     const size_t nl = (size_t)P.npe * P.ncu * ne;
     EXA_TRY(dev_alloc(c, &c.ldg_R, nl));

@@ -8,6 +8,7 @@
 #include "exa_assembly.cuh"
 #include "exa_ldg.cuh"
 #include "exa_ldg_tp.cuh"
+#include "exa_hdg_tp.cuh"
 #include "exa_vol_tp.cuh"
 #include "exa_solver.cuh"
 #include "exa_umma.cuh"
@@ -366,6 +367,11 @@ int exa_model_assemble(ExaCtx& c, bool jacobian) {
   const ExaDims& P = c.P;
   const int n = P.n, m = P.m;
   const long long nqn = (long long)P.npe * P.nd * P.ncu;
+  if (!jacobian && c.tp_nslot) {
+    ExaProfScope ps(c, EXA_PH_RESIDUAL);
+    int rc = EXA_OK;
+    if (launch_hdg_resid_tp<ExaModel>(make_args(c, 0), c.tensor, c.tp_nslot, c.Ru, c.Rh, c.st, &rc)) return rc;
+  }
   const size_t vs = jacobian ? vol_points_smem<true>(P) : vol_points_smem<false>(P);
   const size_t fs = face_smem(P, jacobian);
   if (jacobian) {
@@ -458,6 +464,10 @@ int exa_model_assemble(ExaCtx& c, bool jacobian) {
   return EXA_OK;
 }
 
+bool exa_model_getq_tp(ExaCtx& c, int* rc) {
+  return c.tp_nslot && launch_getq_tp(c.P, c.tensor, c.tp_nslot, c.perm, c.elemcon, c.elemg, c.faceg, c.uh, c.udg, c.st, rc);
+}
+
 bool exa_model_has_ldg_boundary() { return ExaModel::has_ldg_boundary; }
 
 namespace {
@@ -496,7 +506,7 @@ bool ldg_residual_tp(ExaCtx& c, const LdgState& U, double* out, int* rc) {
     Boundary& q = *static_cast<Boundary*>(p);
     return ldg_faces_general(q.c, q.L, q.c.P.nf0);
   };
-  return launch_ldg_tp<ExaModel>(b.L, make_args(c, 0), U, c.tensor, c.ldg_nslot, c.ldg_fslot, out, c.st, boundary, &b,
+  return launch_ldg_tp<ExaModel>(b.L, make_args(c, 0), U, c.tensor, c.tp_nslot, c.ldg_fslot, out, c.st, boundary, &b,
                                  rc);
 }
 

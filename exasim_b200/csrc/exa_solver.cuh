@@ -142,10 +142,11 @@ struct ExaCtx {
   // R(u), a perturbed state, its residual, the face residuals [npf, ncu, nf], R at u - eps v
   double *ldg_R = nullptr, *ldg_w = nullptr, *ldg_Rw = nullptr, *ldg_Rh = nullptr, *ldg_Rm = nullptr;
   int ldg_has_boundary = 0;
-  // tensor-product elements (n1 > 0): the 1D tables, and for the LDG element kernel the face
-  // slots of each node [npe, nd] (-1: none) and of each element's face nodes
+  // tensor-product elements (n1 > 0): the 1D tables, the face nodes a + npf l that each element
+  // node is (at most nd, in order, -1: none) [npe, nd] (null: some node lies on more faces), and
+  // for the LDG element kernel where each element's face nodes find their residuals
   ExaTensor tensor;
-  int *ldg_nslot = nullptr, *ldg_fslot = nullptr;
+  int *tp_nslot = nullptr, *ldg_fslot = nullptr;
   // interior faces are faces [0, nf0) and boundary faces the rest (the pointwise interior-face
   // kernel relies on it)
   int ldg_split = 0;
@@ -171,6 +172,8 @@ long long exa_ctx_estimate_bytes(const double* app, long long napp, const double
 // model-specific steps (instantiated per model)
 int exa_model_assemble(ExaCtx& c, bool jacobian);
 int exa_model_init_udg(ExaCtx& c, double* host_udg);
+// q recovery of tensor-product elements; false where there is no instance (*rc: its status)
+bool exa_model_getq_tp(ExaCtx& c, int* rc);
 // LDG residual (residual.cpp:589-617) of the element states u [npe, ncu, ne] into Ru
 int exa_model_ldg_residual(ExaCtx& c, const double* u, double* Ru);
 // w = (R(u + eps v) - R(u)) / eps around u = udg with R(u) in ldg_R (one-sided differences)
