@@ -1,5 +1,6 @@
 // Context setup from Exasim's input blobs and the C ABI of the solver
 // (declarations and reference citations: include/exasim_b200.h).
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -524,6 +525,17 @@ int exa_ctx_init(ExaCtx& c, const double* app, long long napp, const double* mas
     EXA_TRY(dev_alloc(c, &c.wT, (size_t)c.wT_elems * per));
   }
   if (inv_ws) EXA_TRY(dev_alloc(c, &c.wInv, nb * inv_ws));
+  if (hdg && P.ncq == 0 && P.npf * P.ncu <= 512) {
+    std::vector<int> fk;
+    for (int l = 0; l < P.nfe; ++l) {
+      std::vector<int> one;
+      for (int k = 0; k < P.ncu; ++k)
+        for (int a = 0; a < P.npf; ++a) one.push_back(perm[a + P.npf * l] + P.npe * k);
+      std::sort(one.begin(), one.end());
+      fk.insert(fk.end(), one.begin(), one.end());
+    }
+    EXA_TRY(dev_upload(c, &c.face_k, fk.data(), fk.size()));
+  }
   if ((long long)nb * P.nge * P.npe >= (1LL << 25)) {
     // the chunk-wide GEMMs of the residual: udg and the stage source at the Gauss points, and
     // the integrand's contraction with shapegw (one product each over the whole chunk); small
@@ -542,8 +554,10 @@ int exa_ctx_init(ExaCtx& c, const double* app, long long napp, const double* mas
       EXA_TRY(exa_gemm_tune((int)m, P.npe, kq, nbt, c.st));
       EXA_TRY(exa_gemm_tune((int)m, P.ndf, kq, nbt, c.st));
     }
-    EXA_TRY(exa_gemm_tune((int)n, (int)m, (int)n, nbt, c.st));
-    EXA_TRY(exa_gemm_tune((int)m, (int)m, (int)n, nbt, c.st));
+    if (!c.face_k) {
+      EXA_TRY(exa_gemm_tune((int)n, (int)m, (int)n, nbt, c.st));
+      EXA_TRY(exa_gemm_tune((int)m, (int)m, (int)n, nbt, c.st));
+    }
     if (c.wT) EXA_TRY(exa_gemm_tune(P.npe, P.npe, P.nge, nbt, c.st));  // the FP64 volume products
     // and the element inverse (FP64 D of the plain form)
     EXA_TRY(exa_inverse_tune((int)n, (int)std::min<size_t>(nb, 4096), 1, c.st));

@@ -74,6 +74,8 @@ void exa_add_launches(long long n);
 // (b1, b2) in [0, batch) x [0, batch2), with
 //   A(r, k) = A[r + lda*k + sA*b1 + sA2*b2], B(k, c) = B[k + ldb*c + ...], C(r, c) = C[r + ldc*c + ...].
 // beta == 0 does not read C.
+// With kidx, k runs over a list instead: term k of entry b2 takes column kidx[k + skidx b2] of A and
+// that row of B (operands with the same zero columns and rows, left out); K <= 512.
 struct GemmBatch {
   int M, N, K;
   double alpha, beta;
@@ -81,6 +83,8 @@ struct GemmBatch {
   const double* B; long long ldb, sB, sB2;
   double* C; long long ldc, sC, sC2;
   int batch, batch2;
+  const int* kidx;
+  long long skidx;
 };
 int exa_gemm(const GemmBatch& g, cudaStream_t st);
 // Times the FP64 GEMM's candidate CTA tiles for one shape on scratch blocks and keeps the

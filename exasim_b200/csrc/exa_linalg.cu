@@ -137,11 +137,12 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
 
-template <int TI, int TJ, int WM, int WN, int MB, bool VEC>
+template <int TI, int TJ, int WM, int WN, int MB, bool VEC, bool IDX>
 __global__ void __launch_bounds__(32 * WM * WN, MB) dmma_gemm_kernel(GemmBatch g) {
   constexpr int BM = 16 * TI * WM, BN = 8 * TJ * WN, NT = 32 * WM * WN, W = VEC ? 2 : 1;
+  constexpr int WB = VEC && !IDX ? 2 : 1;  // entries per copy of B: listed rows come one by one
   constexpr int SA = dmma_stride(BM);
-  constexpr int RA = BM / W, KB = GK / W;  // copies per column of A, per column of B
+  constexpr int RA = BM / W, KB = GK / WB;  // copies per column of A, per column of B
   constexpr int LA = (RA * GK + NT - 1) / NT, LB = (KB * BN + NT - 1) / NT;
   extern __shared__ __align__(16) double dsm[];
   double* As = dsm;                    // [GST][GK][SA]
@@ -154,6 +155,11 @@ __global__ void __launch_bounds__(32 * WM * WN, MB) dmma_gemm_kernel(GemmBatch g
   double* C = g.C + b1 * g.sC + b2 * g.sC2;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int wm = warp % WM, wn = warp / WM;
+  __shared__ int ks[IDX ? 512 : 1];
+  if constexpr (IDX) {
+    for (int t = tid; t < g.K; t += NT) ks[t] = g.kidx[t + g.skidx * b2];
+    __syncthreads();
+  }
   const int r0 = tm * BM, c0 = tn * BN;
   const int gq = lane >> 2, tq = lane & 3;
   double acc[TI][TJ][4];
@@ -177,17 +183,17 @@ __global__ void __launch_bounds__(32 * WM * WN, MB) dmma_gemm_kernel(GemmBatch g
       if (RA * GK % NT == 0 || k < GK) {
         const int gr = r0 + r, gk = k0 + k;
         const int nb = gk < g.K ? 8 * min(W, max(0, g.M - gr)) : 0;
-        cp_async<W>(as + k * SA + r, nb ? A + gr + g.lda * gk : A, nb);
+        cp_async<W>(as + k * SA + r, nb ? A + gr + g.lda * (IDX ? ks[gk] : gk) : A, nb);
       }
     }
 #pragma unroll
     for (int q = 0; q < LB; ++q) {
       const int t = tid + NT * q;
-      const int k = t % KB * W, c = t / KB;
+      const int k = t % KB * WB, c = t / KB;
       if (KB * BN % NT == 0 || c < BN) {
         const int gk = k0 + k, gc = c0 + c;
-        const int nb = gc < g.N ? 8 * min(W, max(0, g.K - gk)) : 0;
-        cp_async<W>(bs + c * GSB + k, nb ? B + gk + g.ldb * gc : B, nb);
+        const int nb = gc < g.N ? 8 * min(WB, max(0, g.K - gk)) : 0;
+        cp_async<WB>(bs + c * GSB + k, nb ? B + (IDX ? ks[gk] : gk) + g.ldb * gc : B, nb);
       }
     }
   };
@@ -249,22 +255,19 @@ template <int TI, int TJ, int WM, int WN, int MB>
 int launch_dmma(const GemmBatch& g, cudaStream_t st) {
   constexpr int BM = 16 * TI * WM, BN = 8 * TJ * WN;
   constexpr size_t smem = dmma_smem<TI, TJ, WM, WN>();
-  static_assert(MB * smem <= 227 * 1024, "GEMM tiles exceed shared memory");
+  static_assert(MB * (smem + 3072) <= 228 * 1024, "GEMM tiles exceed shared memory");
   // pairs of entries where every copy then starts on a 16-byte boundary
   const bool vec = ((reinterpret_cast<uintptr_t>(g.A) | reinterpret_cast<uintptr_t>(g.B)) & 15) == 0 &&
                    ((g.lda | g.sA | g.sA2 | g.ldb | g.sB | g.sB2) & 1) == 0;
   dim3 grid((unsigned)(exa_ceil_div(g.M, BM) * exa_ceil_div(g.N, BN)), (unsigned)g.batch, (unsigned)g.batch2);
-  if (vec) {
-    auto kern = dmma_gemm_kernel<TI, TJ, WM, WN, MB, true>;
+  auto run = [&](auto kern) -> int {
     EXA_TRY(exa_allow_smem((const void*)kern, smem));
     kern<<<grid, 32 * WM * WN, smem, st>>>(g);
-  } else {
-    auto kern = dmma_gemm_kernel<TI, TJ, WM, WN, MB, false>;
-    EXA_TRY(exa_allow_smem((const void*)kern, smem));
-    kern<<<grid, 32 * WM * WN, smem, st>>>(g);
-  }
-  EXA_LAUNCH_CHECK();
-  return EXA_OK;
+    EXA_LAUNCH_CHECK();
+    return EXA_OK;
+  };
+  if (g.kidx) return vec ? run(dmma_gemm_kernel<TI, TJ, WM, WN, MB, true, true>) : run(dmma_gemm_kernel<TI, TJ, WM, WN, MB, false, true>);
+  return vec ? run(dmma_gemm_kernel<TI, TJ, WM, WN, MB, true, false>) : run(dmma_gemm_kernel<TI, TJ, WM, WN, MB, false, false>);
 }
 
 long long tiles_cost(int M, int N, int bm, int bn) {
@@ -330,6 +333,10 @@ int exa_gemm(const GemmBatch& g, cudaStream_t st) {
       EXA_TRY(exa_gemm(h, st));
     }
     return EXA_OK;
+  }
+  if (g.kidx && (g.K > 512 || g.N == 1)) {
+    exa_set_error("gemm over a list of k: K = %d, N = %d", g.K, g.N);
+    return EXA_ERR_ARG;
   }
   if (g.N == 1) {
     dim3 grid((unsigned)exa_ceil_div(g.M, 128), (unsigned)g.batch, (unsigned)g.batch2);

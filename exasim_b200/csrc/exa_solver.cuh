@@ -65,6 +65,7 @@ struct ExaCtx {
   // FP64 volume products on the DMMA tensor cores
   double* wT = nullptr;
   int wT_elems = 0;
+  int* face_k = nullptr;   // without q: the element unknowns on each face [npf ncu, nfe], increasing
   double* wInv = nullptr;  // blocked-inverse workspace (n^2 per element) when n exceeds the register kernel
   // Krylov / Newton workspace
   double *V = nullptr, *x = nullptr, *r = nullptr, *w = nullptr, *we = nullptr, *du = nullptr;
