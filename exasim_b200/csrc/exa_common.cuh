@@ -87,6 +87,9 @@ struct GemmBatch {
   long long skidx;
 };
 int exa_gemm(const GemmBatch& g, cudaStream_t st);
+// independent products, in one launch where they are small (writing different entries)
+constexpr int EXA_GEMM_GROUP = 4;
+int exa_gemm_group(const GemmBatch* g, int count, cudaStream_t st);
 // Times the FP64 GEMM's candidate CTA tiles for one shape on scratch blocks and keeps the
 // fastest for this device (an autotuner; exa_gemm uses a padding heuristic for shapes not
 // tuned).  The tile does not change the result.  Not for use inside stream capture.

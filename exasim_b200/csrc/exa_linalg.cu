@@ -137,8 +137,8 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
 
-template <int TI, int TJ, int WM, int WN, int MB, bool VEC, bool IDX>
-__global__ void __launch_bounds__(32 * WM * WN, MB) dmma_gemm_kernel(GemmBatch g) {
+template <int TI, int TJ, int WM, int WN, bool VEC, bool IDX>
+__device__ __forceinline__ void dmma_gemm_tile(const GemmBatch& g, const int bx, const long long b1, const long long b2) {
   constexpr int BM = 16 * TI * WM, BN = 8 * TJ * WN, NT = 32 * WM * WN, W = VEC ? 2 : 1;
   constexpr int WB = VEC && !IDX ? 2 : 1;  // entries per copy of B: listed rows come one by one
   constexpr int SA = dmma_stride(BM);
@@ -148,8 +148,7 @@ __global__ void __launch_bounds__(32 * WM * WN, MB) dmma_gemm_kernel(GemmBatch g
   double* As = dsm;                    // [GST][GK][SA]
   double* Bs = dsm + GST * GK * SA;    // [GST][BN][GSB]
   const int tilesM = (g.M + BM - 1) / BM;
-  const int tm = blockIdx.x % tilesM, tn = blockIdx.x / tilesM;
-  const long long b1 = blockIdx.y, b2 = blockIdx.z;
+  const int tm = bx % tilesM, tn = bx / tilesM;
   const double* A = g.A + b1 * g.sA + b2 * g.sA2;
   const double* B = g.B + b1 * g.sB + b2 * g.sB2;
   double* C = g.C + b1 * g.sC + b2 * g.sC2;
@@ -251,6 +250,24 @@ __global__ void __launch_bounds__(32 * WM * WN, MB) dmma_gemm_kernel(GemmBatch g
     }
 }
 
+template <int TI, int TJ, int WM, int WN, int MB, bool VEC, bool IDX>
+__global__ void __launch_bounds__(32 * WM * WN, MB) dmma_gemm_kernel(GemmBatch g) {
+  dmma_gemm_tile<TI, TJ, WM, WN, VEC, IDX>(g, blockIdx.x, blockIdx.y, blockIdx.z);
+}
+
+// several products of one batch in one launch: blockIdx.z counts (product, second batch entry)
+struct GemmGroup {
+  GemmBatch g[EXA_GEMM_GROUP];
+  int batch2;
+};
+template <int TI, int TJ, int WM, int WN, int MB>
+__global__ void __launch_bounds__(32 * WM * WN, MB) dmma_group_kernel(const __grid_constant__ GemmGroup q) {
+  const GemmBatch& g = q.g[blockIdx.z / q.batch2];
+  constexpr int BM = 16 * TI * WM, BN = 8 * TJ * WN;
+  if ((int)blockIdx.x >= ((g.M + BM - 1) / BM) * ((g.N + BN - 1) / BN)) return;
+  dmma_gemm_tile<TI, TJ, WM, WN, false, false>(g, blockIdx.x, blockIdx.y, blockIdx.z % q.batch2);
+}
+
 template <int TI, int TJ, int WM, int WN, int MB>
 int launch_dmma(const GemmBatch& g, cudaStream_t st) {
   constexpr int BM = 16 * TI * WM, BN = 8 * TJ * WN;
@@ -348,6 +365,32 @@ int exa_gemm(const GemmBatch& g, cudaStream_t st) {
   return launch_tile(gemm_tile(g.M, g.N, g.K), g, st);
 }
 
+// Small products (up to 40 x 40 blocks, where a launch costs more than its work: 512 elements of p = 3
+// triangles took 6 us per product) go in one launch, others one after another.
+int exa_gemm_group(const GemmBatch* g, int count, cudaStream_t st) {
+  bool small = count > 1 && count <= EXA_GEMM_GROUP;
+  for (int i = 0; i < count && small; ++i)
+    small = g[i].M <= 40 && g[i].N <= 40 && g[i].M > 0 && g[i].N > 1 && !g[i].kidx && g[i].batch == g[0].batch &&
+            g[i].batch2 == g[0].batch2;
+  small = small && g[0].batch > 0 && g[0].batch <= 65535 && g[0].batch2 > 0 && (long long)g[0].batch2 * count <= 65535;
+  if (!small) {
+    for (int i = 0; i < count; ++i) EXA_TRY(exa_gemm(g[i], st));
+    return EXA_OK;
+  }
+  GemmGroup q{};
+  int tiles = 1;
+  for (int i = 0; i < count; ++i) {
+    q.g[i] = g[i];
+    tiles = std::max(tiles, exa_ceil_div(g[i].M, 32) * exa_ceil_div(g[i].N, 32));
+  }
+  q.batch2 = g[0].batch2;
+  constexpr size_t smem = dmma_smem<1, 2, 2, 2>();
+  EXA_TRY(exa_allow_smem((const void*)dmma_group_kernel<1, 2, 2, 2, 4>, smem));
+  dmma_group_kernel<1, 2, 2, 2, 4><<<dim3(tiles, g[0].batch, q.batch2 * count), 128, smem, st>>>(q);
+  EXA_LAUNCH_CHECK();
+  return EXA_OK;
+}
+
 // Measures the candidate tiles of an M x N x K product on `batch` scratch blocks (at most
 // 512) and keeps the fastest for this device and shape; later products of that shape use
 // it.  Every tile accumulates each entry over k in the same order, so the choice changes
@@ -420,22 +463,23 @@ constexpr int INV_MAX_N = 160;
 template <typename T>
 __device__ __forceinline__ T absval(T x) { return x < T(0) ? -x : x; }
 
-// n <= 32: one warp per matrix, lane r holding row r.  The pivot search is a warp argmax,
+// n <= NM <= 32: one warp per matrix, lane r holding row r (NM = 8, 16, 24, 32: a step costs NM
+// shuffles and updates whatever n is).  The pivot search is a warp argmax,
 // the pivot row reaches every lane by shuffles.  8 matrices per 256-thread CTA.
-template <typename T>
+template <typename T, int NM>
 __global__ void __launch_bounds__(256) inverse_warp_kernel(T* Aall, int n, long long stride, int batch, int* flag) {
   const int lane = threadIdx.x & 31;
   const long long mat = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (mat >= batch) return;
   T* G = Aall + mat * stride;
-  T a[32];
+  T a[NM];
 #pragma unroll
-  for (int j = 0; j < 32; ++j) a[j] = (lane < n && j < n) ? G[lane + (long long)n * j] : T(0);
+  for (int j = 0; j < NM; ++j) a[j] = (lane < n && j < n) ? G[lane + (long long)n * j] : T(0);
   bool used = lane >= n;
   bool singular = false;
   int mystep = 0, myperm = 0;
 #pragma unroll
-  for (int k = 0; k < 32; ++k) {
+  for (int k = 0; k < NM; ++k) {
     if (k >= n) break;
     T best = used ? T(-1) : absval(a[k]);
     int bi = used ? n : lane;
@@ -456,7 +500,7 @@ __global__ void __launch_bounds__(256) inverse_warp_kernel(T* Aall, int n, long 
     if (lane == k) myperm = p;
     const T f = a[k];
 #pragma unroll
-    for (int j = 0; j < 32; ++j) {
+    for (int j = 0; j < NM; ++j) {
       const T rpd = __shfl_sync(0xffffffffu, a[j], p) * d;   // a_pj d
       if (lane == p) a[j] = (j == k) ? d : rpd;
       else a[j] = (j == k) ? -f * d : a[j] - f * rpd;
@@ -465,7 +509,7 @@ __global__ void __launch_bounds__(256) inverse_warp_kernel(T* Aall, int n, long 
   if (singular && lane == 0) atomicExch(flag, 1);
   // entry (r, c) of the tableau is inverse(pos[r], perm[c]); pos[r] = the step of row r
 #pragma unroll
-  for (int c = 0; c < 32; ++c) {
+  for (int c = 0; c < NM; ++c) {
     const int pc = __shfl_sync(0xffffffffu, myperm, c);
     if (c < n && lane < n) G[mystep + (long long)n * pc] = a[c];
   }
@@ -844,7 +888,12 @@ int inverse_dispatch(T* A, int n, long long stride, int batch, int* d_flag, cuda
   if (n <= 32) {
     for (int b0 = 0; b0 < batch; b0 += 8 * 65535) {
       const int nb = (batch - b0 < 8 * 65535) ? batch - b0 : 8 * 65535;
-      inverse_warp_kernel<T><<<exa_ceil_div(nb, 8), 256, 0, st>>>(A + (long long)b0 * stride, n, stride, nb, d_flag);
+      T* Ab = A + (long long)b0 * stride;
+      const int g = exa_ceil_div(nb, 8);
+      if (n <= 8) inverse_warp_kernel<T, 8><<<g, 256, 0, st>>>(Ab, n, stride, nb, d_flag);
+      else if (n <= 16) inverse_warp_kernel<T, 16><<<g, 256, 0, st>>>(Ab, n, stride, nb, d_flag);
+      else if (n <= 24) inverse_warp_kernel<T, 24><<<g, 256, 0, st>>>(Ab, n, stride, nb, d_flag);
+      else inverse_warp_kernel<T, 32><<<g, 256, 0, st>>>(Ab, n, stride, nb, d_flag);
       EXA_LAUNCH_CHECK();
     }
     return EXA_OK;

@@ -41,7 +41,8 @@ int smem_attr(const void* fn, size_t bytes) {
 // runs on the context's second stream, beside the three products into F, K and H: its pivot
 // loop is latency-bound and the products are HBM- or tensor-bound.  With phase profiling on,
 // everything stays on the context stream, so the phase events time each step alone.
-bool overlap_inverse(const ExaCtx& c) { return c.P.ncq > 0 && c.st2 && !c.prof.on; }
+// Blocks of a warp's inverse (order up to 32) are too short a step to pay for the two events.
+bool overlap_inverse(const ExaCtx& c) { return c.P.ncq > 0 && c.st2 && !c.prof.on && c.P.n > 32; }
 
 // The context stream joins the second stream before any later work, on every path out of a
 // Schur step (an early error return included), so nothing it runs next can overlap it.
@@ -98,31 +99,38 @@ int schur_chunk(ExaCtx& c, int e0, int nb) {
     GemmBatch g{};
     g.batch = nb; g.batch2 = ncu;
     g.K = (int)kq; g.beta = 1.0;
+    GemmBatch q4[EXA_GEMM_GROUP];
     // D(:, j + npe*b) += sum_(l,d) B(:, l + npe*d + npe*nd*b) MinvC(l, d, j)
     g.M = n; g.N = npe; g.alpha = 1.0;
     g.A = c.wB; g.lda = n; g.sA = (long long)n * nqn; g.sA2 = (long long)n * kq;
     g.B = MC; g.ldb = kq; g.sB = kq * npe; g.sB2 = 0;
     g.C = c.wD; g.ldc = n; g.sC = (long long)n * n; g.sC2 = (long long)n * npe;
-    EXA_TRY(exa_gemm(g, c.st));
-    if (overlap) EXA_TRY(inverse_beside(c, join, [&](cudaStream_t s) {
-      return exa_inverse_ws(c.wD, n, (long long)n * n, nb, c.wInv, c.d_flag, s);
-    }));
+    q4[0] = g;
     // F(:, b + ncu*jf) -= sum_(l,d) B(:, l + npe*d + npe*nd*b) MinvE(l, d, jf)
     g.N = ndf; g.alpha = -1.0;
     g.B = ME; g.ldb = kq; g.sB = kq * ndf;
     g.C = c.wF; g.ldc = (long long)n * ncu; g.sC = (long long)n * m; g.sC2 = n;
-    EXA_TRY(exa_gemm(g, c.st));
+    q4[1] = g;
     // K(:, j + npe*b) += sum_(l,d) G(:, l + npe*d + npe*nd*b) MinvC(l, d, j)
     g.M = m; g.N = npe; g.alpha = 1.0;
     g.A = c.wG; g.lda = m; g.sA = (long long)m * nqn; g.sA2 = (long long)m * kq;
     g.B = MC; g.ldb = kq; g.sB = kq * npe;
     g.C = c.wK; g.ldc = m; g.sC = (long long)m * n; g.sC2 = (long long)m * npe;
-    EXA_TRY(exa_gemm(g, c.st));
+    q4[2] = g;
     // H(:, b + ncu*jf) -= sum_(l,d) G(:, l + npe*d + npe*nd*b) MinvE(l, d, jf)
     g.N = ndf; g.alpha = -1.0;
     g.B = ME; g.ldb = kq; g.sB = kq * ndf;
     g.C = Hc; g.ldc = (long long)m * ncu; g.sC = (long long)m * m; g.sC2 = m;
-    EXA_TRY(exa_gemm(g, c.st));
+    q4[3] = g;
+    if (overlap) {
+      EXA_TRY(exa_gemm(q4[0], c.st));
+      EXA_TRY(inverse_beside(c, join, [&](cudaStream_t s) {
+        return exa_inverse_ws(c.wD, n, (long long)n * n, nb, c.wInv, c.d_flag, s);
+      }));
+      for (int i = 1; i < 4; ++i) EXA_TRY(exa_gemm(q4[i], c.st));
+    } else {
+      EXA_TRY(exa_gemm_group(q4, 4, c.st));
+    }
   }
   if (overlap) {
     EXA_TRY(join.join());
@@ -343,6 +351,7 @@ int volume_blocks_gemm(ExaCtx& c, int nb) {
     vol_t_kernel<<<(unsigned)std::min<long long>((tot + 255) / 256, 8192), 256, 0, c.st>>>(P, c.shapegw, c.wRg, le0,
                                                                                          nbs, c.wT);
     EXA_LAUNCH_CHECK();
+    std::vector<GemmBatch> gs;
     for (int cc = 0; cc < P.nc; ++cc) {
       GemmBatch g{};
       g.M = npe; g.N = npe; g.K = nge; g.alpha = 1.0; g.beta = 0.0;
@@ -358,8 +367,10 @@ int volume_blocks_gemm(ExaCtx& c, int nb) {
       }
       g.sC2 = npe;  // trace component k: rows npe k
       g.batch = nbs; g.batch2 = ncu;
-      EXA_TRY(exa_gemm(g, c.st));
+      gs.push_back(g);
     }
+    for (size_t i = 0; i < gs.size(); i += EXA_GEMM_GROUP)
+      EXA_TRY(exa_gemm_group(&gs[i], (int)std::min<size_t>(EXA_GEMM_GROUP, gs.size() - i), c.st));
   }
   return EXA_OK;
 }
