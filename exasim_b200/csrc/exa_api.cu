@@ -514,6 +514,7 @@ int exa_ctx_init(ExaCtx& c, const double* app, long long napp, const double* mas
     EXA_TRY(dev_alloc(c, &c.wG, std::max<size_t>(1, nb * m * nqn)));
     EXA_TRY(dev_alloc(c, &c.wRg, nb * P.nge * (P.nd + 1) * P.ncu * P.nc));
     EXA_TRY(dev_alloc(c, &c.wRu, nb * n));
+    if (exa_model_qelim_tp(c)) EXA_TRY(dev_alloc(c, &c.wFq, nb * 2 * P.nfe * P.ngf * P.ncu * P.ncq));
   }
   EXA_TRY(dev_alloc(c, &c.wUG, nb * P.nge * P.nc));
   EXA_TRY(dev_alloc(c, &c.wSG, nb * P.nge * P.ncu));
@@ -1005,6 +1006,7 @@ int exa_get_field(exa_ctx* h, const char* name, double* host, long long n) {
     exa_set_error("get_field('%s'): unknown name or size %lld != %lld", name ? name : "", n, f.n);
     return EXA_ERR_ARG;
   }
+  if (f.p == h->c.wB) EXA_TRY(exa_model_form_b(h->c));
   EXA_CUDA(cudaStreamSynchronize(h->c.st));
   if (n && f.p32) {
     std::vector<float> t((size_t)n);
@@ -1023,6 +1025,7 @@ int exa_set_field(exa_ctx* h, const char* name, const double* host, long long n)
     exa_set_error("set_field('%s'): unknown name or size %lld != %lld", name ? name : "", n, f.n);
     return EXA_ERR_ARG;
   }
+  if (f.p == h->c.wB) h->c.b_pending = false;
   EXA_CUDA(cudaStreamSynchronize(h->c.st));
   if (n && f.p32) {
     std::vector<float> t(host, host + n);
@@ -1039,6 +1042,10 @@ int exa_field_ptr(exa_ctx* h, const char* name, double** dev, long long* n) {
   if (!field(h->c, name, f) || !dev || !n) {
     exa_set_error("field_ptr('%s'): unknown name", name ? name : "");
     return EXA_ERR_ARG;
+  }
+  if (f.p == h->c.wB) {  // the pointer shows B of every later assembly too
+    EXA_TRY(exa_model_form_b(h->c));
+    h->c.b_given = true;
   }
   *dev = f.p32 ? reinterpret_cast<double*>(f.p32) : f.p;
   *n = f.n;

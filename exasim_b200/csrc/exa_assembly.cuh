@@ -41,6 +41,10 @@ struct AsmArgs {
   // when set, the volume kernel leaves its Ru integrand [nge, nd + 1, ncu] per chunk element
   // here and the contraction with shapegw runs as one GEMM over the chunk
   double* rgout;
+  // when set, the face kernel leaves the derivatives of the face fluxes with respect to q here (per
+  // element [u rows, trace rows][nfe][ngf, ncu, ncq]) and forms the blocks of the u and uhat columns
+  // only: the q elimination applies those of q itself (exa_qelim_tp.cuh)
+  double* fqout;
 };
 
 // ----------------------------------------------------------------------------------
@@ -567,7 +571,15 @@ __global__ void face_kernel(AsmArgs A, double* Ru, double* Rh, double* D, double
       // one thread per face-node pair (a, b): the weight w_g = shapfgw[a, g] shapfgt[g, b] is
       // formed once per g and shared by every column q = k + ncu c, taken QC at a time
       constexpr int QC = 4;
-      const int nq = ncu * nc;
+      const int nq = A.fqout ? ncu * ncu : ncu * nc;
+      if (A.fqout) {
+        const int per = ngf * ncu * (nc - ncu);
+        double* o = A.fqout + ((long long)le * 2 * nfe + l) * per;
+        for (int t = threadIdx.x; t < per; t += blockDim.x) {
+          o[t] = fh_uq[ngf * ncu * ncu + t];
+          o[(long long)nfe * per + t] = fT_uq[ngf * ncu * ncu + t];
+        }
+      }
       const int qg = exa_tc::qk_group(npe);  // K group of the packed B and G
       // the pair products of the face, in TA (FP64, or FP32 in the mixed form)
       auto pairs = [&](auto zero, const auto* W, const auto* Tt, const auto* fq, const auto* fTq, const auto* fh,

@@ -9,6 +9,7 @@
 #include "exa_ldg.cuh"
 #include "exa_ldg_tp.cuh"
 #include "exa_hdg_tp.cuh"
+#include "exa_qelim_tp.cuh"
 #include "exa_vol_tp.cuh"
 #include "exa_solver.cuh"
 #include "exa_umma.cuh"
@@ -78,6 +79,9 @@ int inverse_beside(ExaCtx& c, InverseJoin& j, Fn&& fn) {
   return st;
 }
 
+// the plain form's q elimination by sum factorization (exa_qelim_tp.cuh)
+bool tp_qelim(const ExaCtx& c) { return c.wFq && c.precision != 1; }
+
 // Schur condensation of one chunk (uequation.cpp:559-775): q-elimination, D^-1, DinvF,
 // Ru <- D^-1 Ru, H += K DinvF, Rh -= K Ru.
 int schur_chunk(ExaCtx& c, int e0, int nb) {
@@ -85,9 +89,15 @@ int schur_chunk(ExaCtx& c, int e0, int nb) {
   const int n = P.n, m = P.m, npe = P.npe, nd = P.nd, ncu = P.ncu, ndf = P.ndf;
   const long long nqn = (long long)npe * nd * ncu;
   double* Hc = c.H + (long long)e0 * m * m;
-  const bool overlap = overlap_inverse(c);
+  const bool overlap = overlap_inverse(c) && !tp_qelim(c);
   InverseJoin join{c};
-  if (P.ncq > 0) {
+  if (tp_qelim(c)) {
+    ExaProfScope ps(c, EXA_PH_QELIM);
+    const double* MC = c.MC + (long long)e0 * npe * npe * nd;
+    const double* ME = c.ME + (long long)e0 * npe * ndf * nd;
+    EXA_TRY(launch_qelim_tp(P, c.tensor, c.tp_nslot, c.perm, c.bf + (long long)e0 * P.nfe, c.wRg,
+                                    c.wFq, MC, ME, c.wD, c.wF, c.wK, Hc, nb, c.st));
+  } else if (P.ncq > 0) {
     ExaProfScope ps(c, EXA_PH_QELIM);
     // four GEMMs per trace component with K = npe*nd: (n + m) rows x (npe + ndf) columns in all
     exa_prof_flops(c, EXA_PH_QELIM, 2.0 * nb * ncu * (double)npe * nd * (double)(n + m) * (npe + ndf));
@@ -435,7 +445,7 @@ int exa_model_assemble(ExaCtx& c, bool jacobian) {
         if (packed) {
           EXA_TRY(exa_k_vol_mat_tc(P, c.shapegw32, c.Sp, c.wRg, c.wD, c.wB, bp, nb, c.d_uflag, c.st));
         } else if (exa_tensor_blocks(P, c.tensor) &&
-                   launch_vol_blocks_tp(P, c.tensor, c.wRg, c.wD, c.wB, nb, c.st, &rc)) {
+                   launch_vol_blocks_tp(P, c.tensor, c.wRg, c.wD, c.wB, 0, tp_qelim(c) ? P.ncu : P.nc, nb, c.st, &rc)) {
           EXA_TRY(rc);
         } else if (c.wT) {
           EXA_TRY(volume_blocks_gemm(c, nb));
@@ -454,12 +464,17 @@ int exa_model_assemble(ExaCtx& c, bool jacobian) {
         // lists for every element); the rest is structurally zero.  The plain form's products
         // overwrite these arrays, so it zeroes them each time; in the mixed form the products
         // only read them, and the zeros of the switch to that form (exa_ctx_set_precision) stay.
-        const bool zero_blocks = c.precision != 1;
+        // The tensor-product q elimination reads the face blocks of F, K and H only and assigns every
+        // entry.
+        const bool zero_blocks = c.precision != 1 && !tp_qelim(c);
         if (zero_blocks) {
           EXA_CUDA(cudaMemsetAsync(c.wF, 0, sizeof(double) * (size_t)nb * n * m, c.st));
           EXA_CUDA(cudaMemsetAsync(c.wK, 0, sizeof(double) * (size_t)nb * m * n, c.st));
         }
-        if (nqn > 0 && P.ncq > 0) {
+        if (tp_qelim(c)) {
+          A.fqout = c.wFq;
+          c.b_pending = c.neb == P.ne;
+        } else if (nqn > 0 && P.ncq > 0) {
           if (c.precision == 1 && c.wGp.hi) {
             // G written packed by the face kernel.  Each element slot gets the same entries
             // assigned at every assembly (face l's trace rows against face l's nodes, the same
@@ -475,6 +490,7 @@ int exa_model_assemble(ExaCtx& c, bool jacobian) {
         EXA_LAUNCH_CHECK();
       }
       EXA_TRY(c.precision == 1 ? schur_chunk_mixed(c, e0, nb) : schur_chunk(c, e0, nb));
+      if (c.b_given) EXA_TRY(exa_model_form_b(c));
     } else {
       ExaProfScope ps(c, EXA_PH_RESIDUAL);
       if (c.wRG) EXA_TRY(volume_gauss_values(c, A, e0, nb));
@@ -492,6 +508,23 @@ int exa_model_assemble(ExaCtx& c, bool jacobian) {
 
 bool exa_model_getq_tp(ExaCtx& c, int* rc) {
   return c.tp_nslot && launch_getq_tp(c.P, c.tensor, c.tp_nslot, c.perm, c.elemcon, c.elemg, c.faceg, c.uh, c.udg, c.st, rc);
+}
+
+bool exa_model_qelim_tp(const ExaCtx& c) {
+  return c.tp_nslot && exa_tensor_blocks(c.P, c.tensor) && qelim_tp_fits(c.P, c.tensor);
+}
+
+int exa_model_form_b(ExaCtx& c) {
+  const ExaDims& P = c.P;
+  int rc = EXA_OK;
+  if (!c.b_pending) return EXA_OK;
+  c.b_pending = false;
+  if (!launch_vol_blocks_tp(P, c.tensor, c.wRg, c.wD, c.wB, P.ncu, P.nc, P.ne, c.st, &rc))
+    return EXA_OK;
+  EXA_TRY(rc);
+  face_b_kernel<<<P.ne, 128, 0, c.st>>>(P, c.shapfgt, c.shapfgw, c.perm, c.wFq, c.wB);
+  EXA_LAUNCH_CHECK();
+  return EXA_OK;
 }
 
 bool exa_model_has_ldg_boundary() { return ExaModel::has_ldg_boundary; }

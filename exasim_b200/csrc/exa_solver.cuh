@@ -59,6 +59,9 @@ struct ExaCtx {
   // assembly workspace for a chunk of `neb` elements
   int neb = 0;
   double *wD = nullptr, *wB = nullptr, *wF = nullptr, *wK = nullptr, *wG = nullptr, *wRg = nullptr, *wRu = nullptr;
+  double* wFq = nullptr;  // derivatives of the face fluxes with respect to q (tensor-product q elimination), per chunk
+  bool b_pending = false;  // B of the last assembly is not formed yet (exa_model_form_b)
+  bool b_given = false;    // a caller holds the "B" pointer: every assembly forms it
   // per chunk: udg and sdg at the Gauss points and the Ru integrand (the volume kernel's GEMMs)
   double *wUG = nullptr, *wSG = nullptr, *wRG = nullptr;
   // the volume blocks' left factors T = -(shapegw . rgJ) of up to wT_elems elements, for the
@@ -175,6 +178,10 @@ int exa_model_assemble(ExaCtx& c, bool jacobian);
 int exa_model_init_udg(ExaCtx& c, double* host_udg);
 // q recovery of tensor-product elements; false where there is no instance (*rc: its status)
 bool exa_model_getq_tp(ExaCtx& c, int* rc);
+// whether the q elimination applies B and G by sum factorization (wFq) instead of forming them, and
+// B of the last assembly for callers that read the field
+bool exa_model_qelim_tp(const ExaCtx& c);
+int exa_model_form_b(ExaCtx& c);
 // LDG residual (residual.cpp:589-617) of the element states u [npe, ncu, ne] into Ru
 int exa_model_ldg_residual(ExaCtx& c, const double* u, double* Ru);
 // w = (R(u + eps v) - R(u)) / eps around u = udg with R(u) in ldg_R (one-sided differences)

@@ -42,7 +42,7 @@ struct VolTp {
 // One block per (element, pair).
 template <int ND, int N1>
 __global__ void __launch_bounds__(VTP_T, 2)
-    vol_blocks_tp_kernel(ExaDims P, const double* __restrict__ rgJ, double* __restrict__ D, double* __restrict__ B,
+    vol_blocks_tp_kernel(ExaDims P, int cfirst, const double* __restrict__ rgJ, double* __restrict__ D, double* __restrict__ B,
                          const __grid_constant__ TensorPair<N1> T) {
   using V = VolTp<ND, N1>;
   constexpr int NP = V::NP, Q = V::Q, PR = V::PR, LI = V::LI, GW = V::GW;
@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(VTP_T, 2)
   double* tab = R + (ND + 1) * NP;        // SS, DS: [Q][N1] each
   double* stage = tab + 2 * Q * N1;       // [warps][GW][N1][NP]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int le = blockIdx.y, kc = blockIdx.x, ncu = P.ncu, n = P.n;
+  const int le = blockIdx.y, kc = blockIdx.x + P.ncu * cfirst, ncu = P.ncu, n = P.n;
   const int k = kc % ncu, c = kc / ncu;
   const double* Rg = rgJ + ((long long)le * ncu * P.nc + kc) * (ND + 1) * NP;
   for (int t = tid; t < (ND + 1) * NP; t += VTP_T) R[t] = Rg[t];
@@ -161,16 +161,16 @@ __global__ void __launch_bounds__(VTP_T, 2)
   }
 }
 
-// Launches it where the element's order has an instance; *rc: EXA_OK or the launch's error
-inline bool launch_vol_blocks_tp(const ExaDims& P, const ExaTensor& T, const double* rgJ, double* D, double* B,
-                                 int nb, cudaStream_t st, int* rc) {
+// Launches it for the pairs of fields c0 .. c1 - 1 where the element's order has an instance; *rc: EXA_OK or the launch's error
+inline bool launch_vol_blocks_tp(const ExaDims& P, const ExaTensor& T, const double* rgJ, double* D, double* B, int c0,
+                                 int c1, int nb, cudaStream_t st, int* rc) {
 #define EXA_VTP(ND, N1)                                                                     \
   if (P.nd == ND && T.n1 == N1) {                                                           \
     *rc = [&]() -> int {                                                                    \
       const size_t sm = sizeof(double) * VolTp<ND, N1>::doubles;                            \
       auto kern = vol_blocks_tp_kernel<ND, N1>;                                             \
       EXA_TRY(exa_allow_smem((const void*)kern, sm));                                       \
-      kern<<<dim3(P.ncu * P.nc, nb), VTP_T, sm, st>>>(P, rgJ, D, B, tensor_pair<N1>(T)); \
+      kern<<<dim3(P.ncu * (c1 - c0), nb), VTP_T, sm, st>>>(P, c0, rgJ, D, B, tensor_pair<N1>(T)); \
       EXA_LAUNCH_CHECK();                                                                   \
       return EXA_OK;                                                                        \
     }();                                                                                    \

@@ -1,0 +1,56 @@
+"""q elimination of scalar models on tensor-product hexahedra (csrc/exa_qelim_tp.cuh), from meshes with
+several blocks per element to one, every order with an instance: the eliminated blocks K and H and the
+block B, which is formed when it is read, against the oracle's dense products.
+
+Tolerances: K and B are sums of at most 1e3 terms over tables of rounding 1e-14 of their largest entries:
+1e-11 of the largest entry; H passes through D^-1 of condition 1e3: 2e-11."""
+import numpy as np
+import pytest
+import torch
+
+from exasim_b200 import HDGSolver, build as B, cases
+from oracle.hdg import HDGOracle
+from oracle.models import MODELS
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,p", [(2, 2), (3, 3), (2, 4), (9, 2)])
+def test_eliminated_blocks_match_oracle(tmp_path, n, p):
+    d = str(tmp_path / "datain")
+    B.build(["convdiff3d"])
+    cases.convdiff3d_hex(d, n=n, porder=p, nsteps=1)
+    s, o = HDGSolver(d, "convdiff3d"), HDGOracle(d, MODELS["convdiff3d"]())
+    o.sdg = 40.0 * o.udg[:, :o.ncu]
+    o.sdgg = np.einsum("gj,jce->gec", o.shapegt[:, :, 0], o.sdg)
+    o.time, o.dtfactor = 0.01, 45.0
+    s.set("sdg", o.sdg.ravel(order="F"))
+    s.set_time(o.time, o.dtfactor)
+    rng = np.random.default_rng(p)
+    err = lambda a, b: np.abs(a - np.asarray(b).ravel(order="F")).max() / np.abs(b).max()
+
+    def step():
+        udg = rng.standard_normal(o.udg.shape)
+        uh = rng.standard_normal(o.uh.shape)
+        s.set("udg", udg)
+        s.set("uh", uh)
+        o.udg, o.uh = udg.copy(), uh.copy()
+        s.hdgAssembleLinearSystem()
+        H = o.assemble()[0]
+        b = o._volume(udg)[2] + o._faces(udg, uh)["Dface"][:, :, :, :, 1:]
+        return H, b[:, :, :, 0].transpose(0, 1, 3, 2)
+
+    H, b = step()
+    assert err(s.get("K"), o.K) < 1e-11 and err(s.get("H"), H) < 2e-11
+    assert err(s.get("B"), b) < 1e-11
+    ptr, size = s.field_ptr("B")  # the pointer shows B of each later assembly
+    view = type("View", (), {"__cuda_array_interface__": {"data": (ptr, False), "shape": (size,), "typestr": "<f8",
+                                                          "version": 3}})()
+    H, b = step()
+    torch.cuda.synchronize()
+    assert err(torch.as_tensor(view, device="cuda").cpu().numpy(), b) < 1e-11
+    H, b = step()
+    s.set("B", 2.0 * s.get("B"))
+    assert err(s.get("B"), 2.0 * b) < 1e-11  # what was written is read back
+    assert err(s.get("H"), H) < 2e-11
+    s.close()
