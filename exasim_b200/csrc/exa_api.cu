@@ -1021,6 +1021,7 @@ int exa_get_field(exa_ctx* h, const char* name, double* host, long long n) {
 int exa_set_field(exa_ctx* h, const char* name, const double* host, long long n) {
   EXA_TRY(guard(h));
   FieldRef f{};
+  if (name && std::string(name) == "K") h->c.k_given = true;
   if (!field(h->c, name, f) || !host || n != f.n) {
     exa_set_error("set_field('%s'): unknown name or size %lld != %lld", name ? name : "", n, f.n);
     return EXA_ERR_ARG;
@@ -1039,6 +1040,7 @@ int exa_set_field(exa_ctx* h, const char* name, const double* host, long long n)
 int exa_field_ptr(exa_ctx* h, const char* name, double** dev, long long* n) {
   EXA_TRY(guard(h));
   FieldRef f{};
+  if (name && std::string(name) == "K") h->c.k_given = true;
   if (!field(h->c, name, f) || !dev || !n) {
     exa_set_error("field_ptr('%s'): unknown name", name ? name : "");
     return EXA_ERR_ARG;

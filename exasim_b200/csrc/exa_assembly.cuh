@@ -383,7 +383,8 @@ __global__ void vol_t_kernel(ExaDims P, const double* __restrict__ shapegw, cons
 //   interior formula into Ru, D, B, F; trace rows (Fbou on boundary faces) into
 //   Rh, K, G, H (uequation.cpp:300-487, kokkosimpl.h:1650-1730).
 // JAC = false computes Ru and Rh only (RuEquationElemFaceBlock, uequation.cpp:883-1077).
-// F, K, G, H must be zero on entry; Ru holds the volume part.
+// The entries of F, K, G and H that couple a face with its own nodes are assigned, the others left;
+// Ru holds the volume part.
 // ----------------------------------------------------------------------------------
 template <class Mdl, bool JAC>
 __global__ void face_kernel(AsmArgs A, double* Ru, double* Rh, double* D, double* B, double* F, double* K,

@@ -85,6 +85,7 @@ struct GemmBatch {
   int batch, batch2;
   const int* kidx;
   long long skidx;
+  int cown;  // > 0: C counts as zero outside the columns [cown b2, cown (b2 + 1)) of entry b2
 };
 int exa_gemm(const GemmBatch& g, cudaStream_t st);
 // independent products, in one launch where they are small (writing different entries)

@@ -245,7 +245,8 @@ __device__ __forceinline__ void dmma_gemm_tile(const GemmBatch& g, const int bx,
           if (gc >= g.N) continue;
           double* p = C + gr + g.ldc * gc;
           const double v = g.alpha * acc[i][j][2 * h + x];
-          *p = (g.beta == 0.0) ? v : v + g.beta * (*p);
+          const bool own = g.beta != 0.0 && (g.cown == 0 || gc / g.cown == (int)b2);
+          *p = own ? v + g.beta * (*p) : v;
         }
     }
 }

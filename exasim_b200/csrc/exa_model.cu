@@ -183,9 +183,10 @@ int schur_chunk(ExaCtx& c, int e0, int nb) {
     g.M = ncf; g.K = ncf; g.batch2 = P.nfe;
     g.kidx = c.face_k; g.skidx = ncf;
     g.sA2 = ncf; g.sC2 = ncf;
+    g.cown = ncf;  // the face kernel fills H's diagonal face blocks only
   }
   EXA_TRY(exa_gemm(g, c.st));
-  g.M = m; g.K = n; g.batch2 = 1; g.kidx = nullptr; g.sA2 = g.sC2 = 0;
+  g.M = m; g.K = n; g.batch2 = 1; g.kidx = nullptr; g.sA2 = g.sC2 = 0; g.cown = 0;
   // Rh -= K Ru
   g.N = 1; g.alpha = -1.0;
   g.B = Ruc; g.ldb = n; g.sB = n;
@@ -467,7 +468,10 @@ int exa_model_assemble(ExaCtx& c, bool jacobian) {
         // The tensor-product q elimination reads the face blocks of F, K and H only and assigns every
         // entry.
         const bool zero_blocks = c.precision != 1 && !tp_qelim(c);
-        if (zero_blocks) {
+        // Without q the products read F at those entries only and take H's other blocks as zero
+        // (face_k); K's other entries are never written.  1000 p = 3 hexahedra of the Euler equations:
+        // 5 GB not written, assembly 13.31 -> 12.59 ms.
+        if (zero_blocks && (!c.face_k || c.k_given)) {
           EXA_CUDA(cudaMemsetAsync(c.wF, 0, sizeof(double) * (size_t)nb * n * m, c.st));
           EXA_CUDA(cudaMemsetAsync(c.wK, 0, sizeof(double) * (size_t)nb * m * n, c.st));
         }
@@ -485,7 +489,7 @@ int exa_model_assemble(ExaCtx& c, bool jacobian) {
             EXA_CUDA(cudaMemsetAsync(c.wG, 0, sizeof(double) * (size_t)nb * m * nqn, c.st));
           }
         }
-        if (zero_blocks) EXA_CUDA(cudaMemsetAsync(Hc, 0, sizeof(double) * (size_t)nb * m * m, c.st));
+        if (zero_blocks && !c.face_k) EXA_CUDA(cudaMemsetAsync(Hc, 0, sizeof(double) * (size_t)nb * m * m, c.st));
         face_kernel<ExaModel, true><<<nb, tpb_f, fs, c.st>>>(A, Ruc, Rhc, c.wD, c.wB, c.wF, c.wK, c.wG, Hc);
         EXA_LAUNCH_CHECK();
       }

@@ -68,6 +68,7 @@ struct ExaCtx {
   // FP64 volume products on the DMMA tensor cores
   double* wT = nullptr;
   int wT_elems = 0;
+  bool k_given = false;    // a caller holds or has written the "K" field: its zeros are set again
   int* face_k = nullptr;   // without q: the element unknowns on each face [npf ncu, nfe], increasing
   double* wInv = nullptr;  // blocked-inverse workspace (n^2 per element) when n exceeds the register kernel
   // Krylov / Newton workspace

@@ -54,3 +54,34 @@ def test_eliminated_blocks_match_oracle(tmp_path, n, p):
     assert err(s.get("B"), 2.0 * b) < 1e-11  # what was written is read back
     assert err(s.get("H"), H) < 2e-11
     s.close()
+
+
+@pytest.mark.parametrize("n,p", [(3, 2), (2, 3)])
+def test_blocks_without_q_are_assembled_again(tmp_path, n, p):
+    """Without q only the entries that couple a face with its own nodes are written again by an assembly:
+    H, F and K of a second state, and after a caller wrote into K, against the oracle."""
+    d = str(tmp_path / "datain")
+    B.build(["euler3d"])
+    cases.euler3d_vortex_hex(d, n=n, porder=p, periodic=n > 2)
+    s, o = HDGSolver(d, "euler3d"), HDGOracle(d, MODELS["euler3d"]())
+    o.sdg = 40.0 * o.udg[:, :o.ncu]
+    o.sdgg = np.einsum("gj,jce->gec", o.shapegt[:, :, 0], o.sdg)
+    o.time, o.dtfactor = 0.01, 45.0
+    s.set("sdg", o.sdg.ravel(order="F"))
+    s.set_time(o.time, o.dtfactor)
+    rng = np.random.default_rng(n)
+    u0, h0 = o.udg.copy(), o.uh.copy()
+    err = lambda a, b: np.abs(a - np.asarray(b).ravel(order="F")).max() / np.abs(b).max()
+    for written in (False, False, True):
+        o.udg = u0 * (1 + 1e-2 * rng.standard_normal(u0.shape)) + 1e-3
+        o.uh = h0 * (1 + 1e-2 * rng.standard_normal(h0.shape)) + 1e-3
+        s.set("udg", o.udg)
+        s.set("uh", o.uh)
+        if written:
+            s.set("K", rng.standard_normal(o.K.size))
+        s.hdgAssembleLinearSystem()
+        H, Rh, F, Ru = o.assemble()
+        for name, ref in (("H", H), ("F", F), ("Ru", Ru), ("Rh", Rh)):
+            assert err(s.get(name), ref) < 5e-12, name
+    assert err(s.get("K"), o.K) < 1e-11
+    s.close()
