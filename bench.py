@@ -789,15 +789,15 @@ def run_served(args, device):
     return out
 
 
-# DRAM traffic of the four q-elimination GEMM launches of one FP64 assembly, from one ncu
-# capture (dram__bytes_read.sum + dram__bytes_write.sum) on the 10^3-element mesh of this
-# workload: 4.458 GB for 1000 elements; it scales with the element count (each element's
-# blocks are read once), so per launch and element it is 4.458e9 / 1000 / 4 bytes.
-QELIM_TRAFFIC_PER_ELEMENT_LAUNCH = 4.458e9 / 1000 / 4
-# The same for the mixed form's four 3xTF32 q-elimination launches (umma3_kernel, FP32
-# operands split on chip), one ncu capture on the 10^3 mesh: 0.564, 0.642, 0.709 and 0.721 GB
-# read + written, mean 0.659 GB per launch for 1000 elements (the algorithmic 0.658).
-QELIM_MIXED_TRAFFIC_PER_ELEMENT_LAUNCH = 0.6590e9 / 1000
+# DRAM traffic of the q-elimination launch of one FP64 assembly (qelim3_kernel), from one ncu
+# capture (dram__bytes_read.sum + dram__bytes_write.sum) on an 11^3-element mesh of this
+# workload: 2.326 GB for 1331 elements; it scales with the element count (each element's
+# blocks are read once).
+QELIM_TRAFFIC_PER_ELEMENT = 2.326e9 / 1331
+# The same for the mixed form's q elimination: two 3xTF32 products (umma3_kernel, FP32 operands
+# split on chip), 0.564 and 0.642 GB read + written on the 10^3 mesh, and the trace rows
+# (trace_q_kernel), 0.534 GB on the 9^3 mesh.
+QELIM_MIXED_TRAFFIC_PER_ELEMENT = (0.564e9 + 0.642e9) / 1000 + 0.534e9 / 729
 
 
 def fp64_gemm_peak(torch):
@@ -841,6 +841,18 @@ def qelim_mixed_bytes(sz):
     return (d + f + k + h) * ne
 
 
+def qelim_bytes(sz):
+    """The same without G, as scalar models on hexahedra run: the products D and F as above; the
+    trace rows read MinvC and MinvE, the FP64 flux derivatives and the face blocks of K and H, and
+    write K plain and packed and H plain."""
+    npe, nd, ne = sz["npe"], sz["nd"], sz["ne"]
+    ndf = sz["npf"] * sz["nfe"]
+    kq = npe * nd
+    df = 2 * 4 * npe * kq + 4 * kq * (npe + ndf) + 12 * npe * (npe + ndf)
+    trace = 4 * kq * (npe + ndf) + 8 * ndf * nd + 2 * 8 * ndf * sz["npf"] + 8 * ndf * npe + 4 * ndf * ndf
+    return (df + trace) * ne
+
+
 def autotuned(s):
     """The shapes the project's autotuners chose for this workload (timed on scratch blocks
     when the contexts were created): the element inverse of order n in FP32 and FP64 (shape
@@ -863,38 +875,38 @@ def autotuned(s):
 
 
 def kernel_rooflines(s32, s64, mixed, plain, torch, steps):
-    """roofline: the q-elimination GEMMs of the mixed solve, umma3_kernel on the TF32 tensor
-    cores, HBM-bound, from the phase timers (CUDA events on the solver's stream around each
-    q-elimination region) of the profiled solves that follow the timed ones.  The plain form's
-    FP64 q-elimination (dmma_gemm_kernel) is reported beside it against cuBLAS DGEMM, and the
-    FP32 condensed matvec is timed alone on the solver's stream."""
+    """roofline: the q elimination of the mixed solve, two products of umma3_kernel on the TF32
+    tensor cores and trace_q_kernel, HBM-bound, from the phase timers (CUDA events on the solver's
+    stream around each q-elimination region) of the profiled solves that follow the timed ones.
+    The plain form's FP64 q elimination (qelim3_kernel) is reported beside it against cuBLAS
+    DGEMM, and the FP32 condensed matvec is timed alone on the solver's stream."""
     peaks, src = measured_peaks()
     sz = s32.sizes
     ne, m, N = sz["ne"], sz["m"], sz["ndofuhat"]
     q_ms, q_regions, _ = mixed["prof"]["qelim"]
-    launches = 4 * q_regions
-    qbytes = qelim_mixed_bytes(sz)
+    launches = 3 * q_regions
+    qbytes = qelim_bytes(sz)
     ms_launch = q_ms / max(launches, 1)
-    achieved = qbytes / 4 / (ms_launch * 1e-3) / 1e9 if q_ms > 0 else 0.0
-    roofline = {"kernel": "umma3_kernel (q-elimination GEMMs D += B MinvC, F -= B MinvE, K += G MinvC, "
-                          "H -= G MinvE; 3xTF32 on tcgen05: FP32 operands by cp.async.bulk, split into TF32 "
-                          "hi and lo parts in shared memory)",
+    achieved = qbytes / 3 / (ms_launch * 1e-3) / 1e9 if q_ms > 0 else 0.0
+    roofline = {"kernel": "umma3_kernel (q-elimination GEMMs D += B MinvC, F -= B MinvE; 3xTF32 on tcgen05: FP32 "
+                          "operands by cp.async.bulk, split into TF32 hi and lo parts in shared memory) and "
+                          "trace_q_kernel (K += G MinvC, H -= G MinvE by sum factorization in FP32)",
                 "bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                 "frac": achieved / peaks["hbm_gbs"], "peak_source": src,
-                "algorithmic_bytes_per_launch": qbytes / 4, "ms_per_launch": ms_launch, "launches": launches,
-                "traffic": QELIM_MIXED_TRAFFIC_PER_ELEMENT_LAUNCH * ne,
-                "traffic_source": "ncu dram bytes of the four launches on a 10^3 mesh, mean per launch, scaled by "
+                "algorithmic_bytes_per_launch": qbytes / 3, "dense_products_bytes": qelim_mixed_bytes(sz), "ms_per_launch": ms_launch, "launches": launches,
+                "traffic": QELIM_MIXED_TRAFFIC_PER_ELEMENT / 3 * ne,
+                "traffic_source": "ncu dram bytes of the three launches on smaller meshes, mean per launch, scaled by "
                                   "element count"}
     p_ms, p_regions, p_flops = plain["prof"]["qelim"]
     peak64 = fp64_gemm_peak(torch)
-    pl = 4 * p_regions
+    pl = p_regions
     p_ach = p_flops / (p_ms * 1e-3) / 1e12 if p_ms > 0 else 0.0
-    plain_roof = {"kernel": "dmma_gemm_kernel (FP64 q-elimination GEMMs on the DMMA tensor cores)", "bound": "tensor",
+    plain_roof = {"kernel": "qelim3_kernel (FP64 q elimination by sum factorization)", "bound": "fp64",
                   "achieved": p_ach, "peak": peak64, "unit": "TFLOP/s", "frac": p_ach / peak64,
                   "peak_source": "cuBLAS DGEMM 8192^3 measured in this run (MEASURED_PEAKS.json has no FP64 figure)",
                   "algorithmic_flops_per_launch": p_flops / max(pl, 1), "ms_per_launch": p_ms / max(pl, 1),
-                  "launches": pl, "traffic": QELIM_TRAFFIC_PER_ELEMENT_LAUNCH * ne,
-                  "traffic_source": "ncu dram bytes of the same launches on a 10^3 mesh, scaled by element count"}
+                  "launches": pl, "traffic": QELIM_TRAFFIC_PER_ELEMENT * ne,
+                  "traffic_source": "ncu dram bytes of the same launch on an 11^3 mesh, scaled by element count"}
     def matvec_roof(s, stream, hbytes, what):
         """The condensed matvec timed alone on the solver's stream: H read once (hbytes per
         entry), the gathered input and element output (16 m ne) and the face vector (16 N)."""

@@ -42,8 +42,8 @@ struct AsmArgs {
   // here and the contraction with shapegw runs as one GEMM over the chunk
   double* rgout;
   // when set, the face kernel leaves the derivatives of the face fluxes with respect to q here (per
-  // element [u rows, trace rows][nfe][ngf, ncu, ncq]) and forms the blocks of the u and uhat columns
-  // only: the q elimination applies those of q itself (exa_qelim_tp.cuh)
+  // element [u rows, trace rows][nfe][ngf, ncu, ncq]) and forms no G, and without a packed B no B
+  // either: the q elimination applies those itself (exa_qelim_tp.cuh)
   double* fqout;
 };
 
@@ -417,9 +417,9 @@ __global__ void face_kernel(AsmArgs A, double* Ru, double* Rh, double* D, double
   int* qtab = reinterpret_cast<int*>(fb_uh + ngf * ncu * ncu);  // ncu*nc
   int* brow = qtab + ncu * nc;  // n: row part, then n: groups of the row's tile
   int* grow = brow + 2 * n;     // m, m
-  // JAC in the mixed form (packed G given): the pair products in FP32, from FP32 copies of the
+  // JAC in the mixed form (packed B or G given): the pair products in FP32, from FP32 copies of the
   // face weights (once per element) and of each face's flux derivatives
-  const bool f32 = JAC && A.Gp.hi != nullptr;
+  const bool f32 = JAC && (A.Gp.hi || A.Bp.hi);
   float* sW32 = reinterpret_cast<float*>(grow + 2 * m);  // npf*ngf
   float* sT32 = sW32 + npf * ngf;                        // ngf*npf
   float* fq32 = sT32 + npf * ngf;                        // ngf*ncu*nc: fh_uq
@@ -572,7 +572,7 @@ __global__ void face_kernel(AsmArgs A, double* Ru, double* Rh, double* D, double
       // one thread per face-node pair (a, b): the weight w_g = shapfgw[a, g] shapfgt[g, b] is
       // formed once per g and shared by every column q = k + ncu c, taken QC at a time
       constexpr int QC = 4;
-      const int nq = A.fqout ? ncu * ncu : ncu * nc;
+      const int nq = A.fqout && !A.Bp.hi ? ncu * ncu : ncu * nc;
       if (A.fqout) {
         const int per = ngf * ncu * (nc - ncu);
         double* o = A.fqout + ((long long)le * 2 * nfe + l) * per;
@@ -653,7 +653,7 @@ __global__ void face_kernel(AsmArgs A, double* Ru, double* Rh, double* D, double
                   } else {
                     A.Gp.hi[o] = (float)vT[u];  // FP32 operand, split by the GEMM on chip
                   }
-                } else {
+                } else if (!A.fqout) {
                   Ge[row_t + (long long)m * col] = vT[u];
                 }
               }

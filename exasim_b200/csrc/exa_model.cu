@@ -81,6 +81,8 @@ int inverse_beside(ExaCtx& c, InverseJoin& j, Fn&& fn) {
 
 // the plain form's q elimination by sum factorization (exa_qelim_tp.cuh)
 bool tp_qelim(const ExaCtx& c) { return c.wFq && c.precision != 1; }
+// its trace rows in the mixed form (B is packed there by the volume kernel)
+bool tp_trace(const ExaCtx& c) { return c.wFq && c.precision == 1 && c.Sp.hi; }
 
 // Schur condensation of one chunk (uequation.cpp:559-775): q-elimination, D^-1, DinvF,
 // Ru <- D^-1 Ru, H += K DinvF, Rh -= K Ru.
@@ -93,6 +95,7 @@ int schur_chunk(ExaCtx& c, int e0, int nb) {
   InverseJoin join{c};
   if (tp_qelim(c)) {
     ExaProfScope ps(c, EXA_PH_QELIM);
+    exa_prof_flops(c, EXA_PH_QELIM, 2.0 * nb * (qelim_tp_volume(c.tensor) + qelim_tp_faces(c.tensor)) * (npe + ndf));
     const double* MC = c.MC + (long long)e0 * npe * npe * nd;
     const double* ME = c.ME + (long long)e0 * npe * ndf * nd;
     EXA_TRY(launch_qelim_tp(P, c.tensor, c.tp_nslot, c.perm, c.bf + (long long)e0 * P.nfe, c.wRg,
@@ -239,7 +242,8 @@ int schur_chunk_mixed(ExaCtx& c, int e0, int nb) {
       EXA_TRY(exa_pack(c.wB, 1, 1, n, (long long)n * nqn, (long long)n * kq, nb, ncu, c.wBp, c.st, kg, npe));
     }
     ExaProfScope ps(c, EXA_PH_QELIM);
-    exa_prof_flops(c, EXA_PH_QELIM, 2.0 * nb * ncu * (double)npe * nd * (double)(n + m) * (npe + ndf));
+    exa_prof_flops(c, EXA_PH_QELIM, tp_trace(c) ? 2.0 * nb * (npe + ndf) * ((double)npe * nd * n + qelim_tp_faces(c.tensor))
+                                                : 2.0 * nb * ncu * (double)npe * nd * (double)(n + m) * (npe + ndf));
     UGemmP u{};
     u.batch = nb; u.batch2 = ncu; u.K = kg * nd; u.beta = 1.0;
     u.tci = EXA_T_F64; u.tco = EXA_T_F32;
@@ -262,6 +266,10 @@ int schur_chunk_mixed(ExaCtx& c, int e0, int nb) {
     toF.cmul = ncu; toF.cadd = 1;
     u.out[0] = toF; u.nout = 1;
     EXA_TRY(exa_gemm_3xtf32(u, c.d_uflag, c.st));
+    // K and H: G is applied from the flux derivatives where the elements are tensor products
+    if (tp_trace(c))
+      EXA_TRY(launch_trace_q(P, c.tensor, c.tp_nslot, c.perm, c.wFq, at(c.MCp, e0), at(c.MEp, e0), c.wK, Hc, K32, H32,
+                             c.Kp, nb, c.st));
     // K(:, j + npe*b) = K + G_b MinvC, plain and packed (A operand of K D^-1 F)
     u.M = m; u.N = npe; u.alpha = 1.0;
     u.A = c.wGp; u.B = at(c.MCp, e0); u.B.sb2 = 0;
@@ -269,14 +277,14 @@ int schur_chunk_mixed(ExaCtx& c, int e0, int nb) {
     u.C = K32; u.ldc = m; u.sC = (long long)m * n; u.sC2 = (long long)m * npe;
     toK.cmul = 1; toK.cadd = npe;
     u.out[0] = toK; u.nout = 1;
-    EXA_TRY(exa_gemm_3xtf32(u, c.d_uflag, c.st));
+    if (!tp_trace(c)) EXA_TRY(exa_gemm_3xtf32(u, c.d_uflag, c.st));
     // H(:, b + ncu*jf) = H - G_b MinvE
     u.N = ndf; u.alpha = -1.0;
     u.B = at(c.MEp, e0); u.B.sb2 = 0;
     u.Cin = Hc; u.ldci = (long long)m * ncu; u.sCi = (long long)m * m; u.sCi2 = m;
     u.C = H32; u.ldc = (long long)m * ncu; u.sC = (long long)m * m; u.sC2 = m;
     u.nout = 0;
-    EXA_TRY(exa_gemm_3xtf32(u, c.d_uflag, c.st));
+    if (!tp_trace(c)) EXA_TRY(exa_gemm_3xtf32(u, c.d_uflag, c.st));
   } else {
     EXA_TRY(exa_k_to_f32(c.wD, D32, (long long)nb * n * n, c.st));
     EXA_TRY(exa_k_to_f32(c.wK, K32, (long long)nb * m * n, c.st));
@@ -478,6 +486,8 @@ int exa_model_assemble(ExaCtx& c, bool jacobian) {
         if (tp_qelim(c)) {
           A.fqout = c.wFq;
           c.b_pending = c.neb == P.ne;
+        } else if (tp_trace(c)) {
+          A.fqout = c.wFq;
         } else if (nqn > 0 && P.ncq > 0) {
           if (c.precision == 1 && c.wGp.hi) {
             // G written packed by the face kernel.  Each element slot gets the same entries

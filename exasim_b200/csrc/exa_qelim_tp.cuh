@@ -10,9 +10,12 @@
 // them.  Bound: the instructions around the products (shared-memory passes and their addresses: FP64
 // units active a quarter of the time).  Measured (B200, 1331 hexahedra, p = 4; before: DMMA products):
 // 4.6 ms with the passes that write B and G -> 2.24 ms, whole assembly 7.37 -> 4.97 ms.  The mixed
-// form keeps its tensor-core products (3.0 ms on 4096 hexahedra, this kernel 6.5).
+// form keeps its tensor-core products into D and F (the four took 3.0 ms on 4096 hexahedra, this kernel
+// 6.5) and has a kernel of its own for the trace rows.
 #pragma once
 #include "exa_hdg_tp.cuh"
+#include "exa_tc.cuh"
+#include "exa_umma.cuh"
 #include "exa_vol_tp.cuh"
 
 // Whole planes in registers: a thread takes both in-plane dimensions of a field's plane or of a face
@@ -276,6 +279,9 @@ __global__ void __launch_bounds__((Qelim3<N1>::NT), 2)
   }
 }
 
+// products per column: the volume part, and the faces'
+inline double qelim_tp_volume(const ExaTensor& T) { return (18.0 * T.n1 + 12.0) * T.n1 * T.n1 * T.n1; }
+inline double qelim_tp_faces(const ExaTensor& T) { return (48.0 * T.n1 + 18.0) * T.n1 * T.n1; }
 // whether a model with q on these elements has an instance
 inline bool qelim_tp_fits(const ExaDims& P, const ExaTensor& T) {
   return P.ncq == 3 && P.nd == 3 && P.ncu == 1 && P.nfe == 6 && T.n1 >= 3 && T.n1 <= 5;
@@ -296,6 +302,207 @@ inline int launch_qelim_tp(const ExaDims& P, const ExaTensor& T, const int* nslo
   }
   EXA_Q3(3) EXA_Q3(4) EXA_Q3(5)
 #undef EXA_Q3
+  exa_set_error("q elimination: no tensor-product instance");
+  return EXA_ERR_UNSUPPORTED;
+}
+
+// The same for the trace rows alone in the mixed form: K = K + G MinvC and H = H - G MinvE in FP32,
+//   G x = Sw (x) Sw sum_d f_d (S (x) S) x_d   on the nodes of each face,
+// in place of products with G, whose rows meet the nodes of one face only (75 of 375 columns at p = 4)
+// and whose 150 rows fill two tensor-core tiles of 128.  One warp per face, one column of MinvC or
+// MinvE per lane, a face's plane in registers, the 1D tables in constant memory: 1075 products per face
+// and column against 9.4 thousand.  Bound: instructions and the latency of the loads (2.9 GB, 0.44 ms at
+// the copy rate).  Measured (B200, 4096 hexahedra, p = 4; before: two 3xTF32 products): 1.87 -> 0.90 ms,
+// and 0.15 ms in the face kernel, which writes no G; the assembly 8.70 -> 7.64 ms.  Three blocks per SM
+// instead of four: 1.10 ms.  Without the prefetch of the columns 64 elements on the assembly takes
+// 7.69 ms.
+constexpr int TRQ_COLS = 32, TRQ_LD = 34;  // columns of a block; row stride (its quads land in other banks)
+constexpr int TRQ_AHEAD = 64;
+template <int N1>
+struct TraceTables {
+  float S[N1 * N1], Sw[N1 * N1];
+};
+template <int N1>
+__global__ void __launch_bounds__(192, 4)
+    trace_q_kernel(ExaDims P, int kg, const int* nslot, const int* perm, const double* __restrict__ Fq, UPacked MC,
+                   UPacked ME, const double* __restrict__ K, const double* __restrict__ H, float* K32, float* H32,
+                   UPacked Kp, const __grid_constant__ TraceTables<N1> T) {
+  constexpr int NP = N1 * N1 * N1, NPF = N1 * N1, M = 6 * NPF, MR = M | 1, FP = (N1 + 3) / 4 * 4;
+  extern __shared__ __align__(16) float xs[];  // [3 kg, whole chunks][TRQ_LD], then the results [TRQ_COLS][MR]
+  __shared__ __align__(16) float sf[6][3][N1][FP];  // derivatives of the trace flux at the points [x][y]
+  __shared__ int sp[M];                        // rows of xs of the face nodes
+  __shared__ unsigned char son[NP];            // faces each node lies on
+  const int le = blockIdx.y, tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+  const int cblocks = (NP + TRQ_COLS - 1) / TRQ_COLS;
+  const bool trace = (int)blockIdx.x >= cblocks;  // columns of MinvE
+  const int c0 = (trace ? blockIdx.x - cblocks : blockIdx.x) * TRQ_COLS;
+  const int ncol = min(TRQ_COLS, (trace ? M : NP) - c0);
+  const UPacked X = trace ? ME : MC;
+  {
+    const float* src = X.hi + (long long)le * X.sb;
+    const int ng = (X.R + 7) / 8, g0 = c0 >> 3;
+    const int blocks = (3 * kg + exa_tc::PK - 1) / exa_tc::PK * 4;
+    float* dl = xs + 4 * (lane >> 3) * TRQ_LD + (lane & 7);
+#pragma unroll 4
+    for (int b = w; b < blocks; b += 6) {  // 8 columns x 16 k, 512 contiguous bytes
+      const int g = b & 3, kb = b >> 2;
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (g0 + g < ng) v = *reinterpret_cast<const float4*>(src + (kb * ng + g0 + g) * 128 + 4 * lane);
+      float* d = dl + 16 * kb * TRQ_LD + 8 * g;
+      d[0] = v.x;
+      d[TRQ_LD] = v.y;
+      d[2 * TRQ_LD] = v.z;
+      d[3 * TRQ_LD] = v.w;
+    }
+    // the columns of the same block TRQ_AHEAD elements on into L2
+    if (le + TRQ_AHEAD < (int)gridDim.y) {
+      const float* nx = src + TRQ_AHEAD * X.sb;
+      for (int t = tid; t < blocks * 4; t += 192) {
+        const int b = t >> 2, g = b & 3, kb = b >> 2;
+        if (g0 + g < ng)
+          asm volatile("prefetch.global.L2 [%0];\n" ::"l"(nx + (kb * ng + g0 + g) * 128 + 32 * (t & 3)));
+      }
+    }
+    const double* fq = Fq + (long long)le * 2 * M * 3 + M * 3;
+    for (int t = tid; t < M * 3; t += 192) {
+      const int l = t / (3 * NPF), d = t / NPF % 3, p = t % NPF;
+      sf[l][d][p % N1][p / N1] = (float)fq[t];
+    }
+    for (int t = tid; t < M; t += 192) sp[t] = perm[t] * TRQ_LD;
+    for (int i = tid; i < NP; i += 192) {
+      int mask = 0;
+      for (int c = 0; c < 3; ++c)
+        if (nslot[3 * i + c] >= 0) mask |= 1 << (nslot[3 * i + c] / NPF);
+      son[i] = (unsigned char)mask;
+    }
+  }
+  __syncthreads();
+  float acc[N1][N1];
+#pragma unroll
+  for (int y = 0; y < N1; ++y)
+#pragma unroll
+    for (int x = 0; x < N1; ++x) acc[y][x] = 0.f;
+  int at[NPF];
+#pragma unroll
+  for (int i = 0; i < NPF; ++i) at[i] = sp[w * NPF + i];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const float* xd = xs + d * kg * TRQ_LD + lane;
+    float a[N1][N1];
+#pragma unroll
+    for (int y = 0; y < N1; ++y) {  // the first dimension of the face, row by row
+      float in[N1];
+#pragma unroll
+      for (int x = 0; x < N1; ++x) in[x] = xd[at[N1 * y + x]];
+#pragma unroll
+      for (int g = 0; g < N1; ++g) {
+        float o = 0.f;
+#pragma unroll
+        for (int x = 0; x < N1; ++x) o = fmaf(T.S[g + N1 * x], in[x], o);
+        a[y][g] = o;
+      }
+    }
+#pragma unroll
+    for (int x = 0; x < N1; ++x) {
+      __align__(16) float f[FP];
+#pragma unroll
+      for (int i = 0; i < FP; i += 4) *reinterpret_cast<float4*>(f + i) = *reinterpret_cast<const float4*>(&sf[w][d][x][i]);
+#pragma unroll
+      for (int g = 0; g < N1; ++g) {
+        float o = 0.f;
+#pragma unroll
+        for (int y = 0; y < N1; ++y) o = fmaf(T.S[g + N1 * y], a[y][x], o);
+        acc[g][x] = fmaf(f[g], o, acc[g][x]);
+      }
+    }
+  }
+  // back to the nodes
+  float out[N1][N1];
+#pragma unroll
+  for (int y = 0; y < N1; ++y)
+#pragma unroll
+    for (int x = 0; x < N1; ++x) {
+      float o = 0.f;
+#pragma unroll
+      for (int g = 0; g < N1; ++g) o = fmaf(T.Sw[g + N1 * x], acc[y][g], o);
+      out[y][x] = o;
+    }
+  __syncthreads();  // the columns have been read: the results take their place
+#pragma unroll
+  for (int x = 0; x < N1; ++x)
+#pragma unroll
+    for (int y = 0; y < N1; ++y) {
+      float o = 0.f;
+#pragma unroll
+      for (int g = 0; g < N1; ++g) o = fmaf(T.Sw[g + N1 * y], out[g][x], o);
+      xs[lane * MR + w * NPF + N1 * y + x] = o;
+    }
+  __syncthreads();
+  // a column per warp; an entry that couples a face with its own nodes adds to what the face kernel left
+  if (trace) {
+    for (int j = w; j < ncol; j += 6) {
+      const int cf = c0 + j, r0 = cf / NPF * NPF;
+      const long long o = (long long)le * M * M + (long long)M * cf;
+#pragma unroll
+      for (int i = 0; i < (M + 31) / 32; ++i) {
+        const int r = lane + 32 * i;
+        if (r >= M) break;
+        const float v = xs[j * MR + r];
+        H32[o + r] = r >= r0 && r < r0 + NPF ? (float)(H[o + r] - (double)v) : -v;
+      }
+    }
+    return;
+  }
+  for (int j = w; j < ncol; j += 6) {
+    const int mask = son[c0 + j];
+    const long long o = (long long)le * M * NP + (long long)M * (c0 + j);
+#pragma unroll
+    for (int i = 0; i < (M + 31) / 32; ++i) {
+      const int r = lane + 32 * i;
+      if (r >= M) break;
+      float v = xs[j * MR + r];
+      if ((mask >> (r / NPF)) & 1) xs[j * MR + r] = v = (float)(K[o + r] + (double)v);
+      K32[o + r] = v;
+    }
+  }
+  __syncthreads();
+  // the packed operand of K D^-1 F, row r and k = column: 8 rows x 4 columns per warp
+  const int nkc = (Kp.K + exa_tc::PK - 1) / exa_tc::PK, ng0 = (min(M, Kp.TR) + 7) / 8, ng1 = (M - Kp.TR + 7) / 8;
+  float* kp = Kp.hi + (long long)le * Kp.sb + lane;
+  const int k3 = lane & 3, r7 = lane >> 2;
+  for (int b = w; b < (M + 7) / 8 * (TRQ_COLS / 4); b += 6) {
+    const int q = b & (TRQ_COLS / 4 - 1), r8 = b / (TRQ_COLS / 4), r = 8 * r8 + r7, k = 4 * q + k3, kk = c0 + 4 * q;
+    if (r >= M || k >= ncol) continue;
+    const int base = 8 * r8 >= Kp.TR ? (Kp.TR / 8) * nkc * 128 + ((kk >> 4) * ng1 + r8 - Kp.TR / 8) * 128
+                                     : ((kk >> 4) * ng0 + r8) * 128;
+    kp[base + ((kk >> 2) & 3) * 32] = xs[k * MR + r];
+  }
+}
+inline size_t trace_q_smem(const ExaDims& P, int kg) {
+  return sizeof(float) * std::max((size_t)(3 * kg + exa_tc::PK - 1) / exa_tc::PK * exa_tc::PK * TRQ_LD, (size_t)TRQ_COLS * (P.m | 1));
+}
+inline int launch_trace_q(const ExaDims& P, const ExaTensor& T, const int* nslot, const int* perm, const double* Fq,
+                          const UPacked& MC, const UPacked& ME, const double* K, const double* H, float* K32, float* H32,
+                          const UPacked& Kp, int nb, cudaStream_t st) {
+  const int kg = exa_tc::qk_group(P.npe);
+  const int blocks = exa_ceil_div(P.npe, TRQ_COLS) + exa_ceil_div(P.ndf, TRQ_COLS);
+  const size_t sm = trace_q_smem(P, kg);
+#define EXA_TRQ(N1)                                                                                                 \
+  if (T.n1 == N1) {                                                                                                 \
+    TraceTables<N1> t;                                                                                              \
+    const Tensor1D<N1> d = tensor_1d<N1>(T);                                                                        \
+    for (int i = 0; i < N1 * N1; ++i) {                                                                             \
+      t.S[i] = (float)d.S[i];                                                                                       \
+      t.Sw[i] = (float)d.Sw[i];                                                                                     \
+    }                                                                                                               \
+    auto kern = trace_q_kernel<N1>;                                                                                 \
+    EXA_TRY(exa_allow_smem((const void*)kern, sm));                                                                 \
+    kern<<<dim3(blocks, nb), 192, sm, st>>>(P, kg, nslot, perm, Fq, MC, ME, K, H, K32, H32, Kp, t);                 \
+    EXA_LAUNCH_CHECK();                                                                                             \
+    return EXA_OK;                                                                                                  \
+  }
+  EXA_TRQ(3) EXA_TRQ(4) EXA_TRQ(5)
+#undef EXA_TRQ
   exa_set_error("q elimination: no tensor-product instance");
   return EXA_ERR_UNSUPPORTED;
 }

@@ -85,3 +85,32 @@ def test_blocks_without_q_are_assembled_again(tmp_path, n, p):
             assert err(s.get(name), ref) < 5e-12, name
     assert err(s.get("K"), o.K) < 1e-11
     s.close()
+
+
+@pytest.mark.parametrize("n,p", [(2, 2), (3, 3), (2, 4), (3, 4)])
+def test_mixed_blocks_match_oracle(tmp_path, n, p):
+    """K and H of the mixed form, whose trace rows are eliminated face by face in FP32 (rounding 6e-8 of
+    sums that cancel to a tenth: 5e-6), H behind a D^-1 of condition 1e3 (2e-4)."""
+    d = str(tmp_path / "datain")
+    B.build(["convdiff3d"])
+    cases.convdiff3d_hex(d, n=n, porder=p, nsteps=1)
+    s, o = HDGSolver(d, "convdiff3d"), HDGOracle(d, MODELS["convdiff3d"]())
+    s.set_precision(1)
+    o.sdg = 40.0 * o.udg[:, :o.ncu]
+    o.sdgg = np.einsum("gj,jce->gec", o.shapegt[:, :, 0], o.sdg)
+    o.time, o.dtfactor = 0.01, 45.0
+    s.set("sdg", o.sdg.ravel(order="F"))
+    s.set_time(o.time, o.dtfactor)
+    rng = np.random.default_rng(p)
+    o.udg, o.uh = rng.standard_normal(o.udg.shape), rng.standard_normal(o.uh.shape)
+    err = lambda a, b: np.abs(a - np.asarray(b).ravel(order="F")).max() / np.abs(b).max()
+    for _ in range(2):
+        s.set("udg", o.udg)
+        s.set("uh", o.uh)
+        s.hdgAssembleLinearSystem()
+        H, Rh, F, Ru = o.assemble()
+        e = {k: err(s.get(k), v) for k, v in (("K32", o.K), ("H32", H), ("F32", F), ("Rh", Rh))}
+        print(n, p, e)
+        assert e["K32"] < 5e-6 and max(e["H32"], e["F32"], e["Rh"]) < 2e-4
+        o.udg = rng.standard_normal(o.udg.shape)
+    s.close()
