@@ -462,7 +462,7 @@ namespace {
 constexpr int INV_MAX_N = 160;
 
 template <typename T>
-__device__ __forceinline__ T absval(T x) { return x < T(0) ? -x : x; }
+__device__ __forceinline__ T absval(T x) { return fabs(x); }  // -0 becomes 0: the pivot search compares bits
 
 // n <= NM <= 32: one warp per matrix, lane r holding row r (NM = 8, 16, 24, 32: a step costs NM
 // shuffles and updates whatever n is).  The pivot search is a warp argmax,

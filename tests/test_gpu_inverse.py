@@ -94,6 +94,27 @@ def test_singular_block_sets_flag(lib, n):
     assert int(flag.item()) == 1
 
 
+@pytest.mark.parametrize("n", [8, 25, 32, 64, 96, 128, 129, 135, 150, 160])
+@pytest.mark.parametrize("fp32", [False, True])
+def test_negative_zeros_are_no_pivots(lib, n, fp32):
+    """Rows of a diagonal matrix in any order with -0 beside the entries (a product of a zero and a negative
+    number): the pivot of each column is its one entry, not a -0, and the inverse is exact."""
+    import torch
+    rng = np.random.default_rng(n)
+    A = np.full((5, n, n), -0.0)
+    for M in A:
+        M[rng.permutation(n), np.arange(n)] = 2.0 ** rng.integers(-3, 4, n) * rng.choice([-1.0, 1.0], n)
+    ref = np.linalg.inv(A)
+    dt, inv = (torch.float32, lib.exa_sinverse_batched) if fp32 else (torch.float64, lib.exa_dinverse_batched)
+    dev = torch.tensor(np.ascontiguousarray(np.transpose(A, (0, 2, 1))).ravel(), dtype=dt, device="cuda")
+    flag = torch.zeros(1, dtype=torch.int32, device="cuda")
+    st = inv(ctypes.c_void_p(dev.data_ptr()), n, n * n, 5, ctypes.c_void_p(flag.data_ptr()), None)
+    assert st == 0, lib.exa_last_error().decode()
+    torch.cuda.synchronize()
+    got = np.transpose(dev.cpu().numpy().reshape(5, n, n), (0, 2, 1))
+    assert int(flag.item()) == 0 and np.array_equal(got, ref)
+
+
 @pytest.mark.parametrize("fp64", [0, 1])
 def test_every_tuned_shape_gives_the_same_bits(lib, fp64):
     """exa_inverse_autotune picks one of the column-by-warp shapes per order; whatever it
