@@ -498,7 +498,7 @@ int exa_ctx_init(ExaCtx& c, const double* app, long long napp, const double* mas
     EXA_TRY(dev_alloc(c, &c.Pc, ne * m * m));
   }
   // element chunk: bounded workspace (about 8 GB at most)
-  const size_t inv_ws = hdg && exa_inverse_needs_ws((int)n) ? n * n : 0;
+  const size_t inv_ws = hdg ? exa_inverse_ws_size((int)n) : 0;
   const size_t vol_ws = (size_t)P.nge * P.nc + (size_t)P.nge * P.ncu + (size_t)P.nge * (P.nd + 1) * P.ncu;
   const size_t per_elem = hdg ? sizeof(double) * (n * n + n * nqn + n * m + m * n + m * nqn +
                                                   (size_t)P.nge * (P.nd + 1) * P.ncu * P.nc + n + inv_ws)
@@ -1368,15 +1368,15 @@ extern "C" int exa_sinverse_batched(float* A, int n, long long stride, int batch
 }
 
 extern "C" int exa_dinverse_batched(double* A, int n, long long stride, int batch, int* info_dev, void* stream) {
-  if (!exa_inverse_needs_ws(n) || batch <= 0) return exa_inverse(A, n, stride, batch, info_dev, (cudaStream_t)stream);
+  if (exa_inverse_ws_size(n) == 0 || batch <= 0) return exa_inverse(A, n, stride, batch, info_dev, (cudaStream_t)stream);
   if (n > exa_inverse_max_n()) {
     exa_set_error("dense inverse of order %d exceeds %d", n, exa_inverse_max_n());
     return EXA_ERR_UNSUPPORTED;
   }
-  // blocked orders: a temporary workspace of n^2 per matrix, freed after the stream drains
+  // blocked orders: a temporary workspace, freed after the stream drains
   cudaStream_t st = (cudaStream_t)stream;
   double* ws = nullptr;
-  EXA_CUDA(cudaMallocAsync((void**)&ws, sizeof(double) * (size_t)n * n * batch, st));
+  EXA_CUDA(cudaMallocAsync((void**)&ws, sizeof(double) * exa_inverse_ws_size(n) * batch, st));
   const int s = exa_inverse_ws(A, n, stride, batch, ws, info_dev, st);
   cudaFreeAsync(ws, st);
   return s;

@@ -109,10 +109,9 @@ int exa_gemm_tile_of(int M, int N, int K);  // index of the tile exa_gemm uses f
 int exa_inverse(double* A, int n, long long stride, int batch, int* d_flag, cudaStream_t st);
 int exa_inverse(float* A, int n, long long stride, int batch, int* d_flag, cudaStream_t st);
 // The same for n up to exa_inverse_max_n(): orders above the register kernel's limit
-// (exa_inverse_needs_ws) are inverted blockwise and need ws, n^2 entries per matrix,
-// spaced n^2 apart.
+// are inverted blockwise and need ws, exa_inverse_ws_size(n) entries per matrix (0: none).
 int exa_inverse_max_n();
-int exa_inverse_needs_ws(int n);
+size_t exa_inverse_ws_size(int n);
 int exa_inverse_ws(double* A, int n, long long stride, int batch, double* ws, int* d_flag, cudaStream_t st);
 int exa_inverse_ws(float* A, int n, long long stride, int batch, float* ws, int* d_flag, cudaStream_t st);
 // FP32 blocks of order up to exa_inverse_max_n(): above the register kernel's limit by the

@@ -461,6 +461,13 @@ int exa_gemm_tile_of(int M, int N, int K) { return gemm_tile(M, N, K); }
 namespace {
 constexpr int INV_MAX_N = 160;
 
+// a subset of a batch: the matrices with only[b] != 0 (null: all), and the stride of the singular
+// flags (0: one flag for the batch, 1: one per matrix)
+struct InvMask {
+  const int* only = nullptr;
+  int fs = 0;
+};
+
 template <typename T>
 __device__ __forceinline__ T absval(T x) { return fabs(x); }  // -0 becomes 0: the pivot search compares bits
 
@@ -525,7 +532,8 @@ __global__ void __launch_bounds__(256) inverse_warp_kernel(T* Aall, int n, long 
 // suffices.
 template <typename T, int TY, int RR, int RC>
 __global__ void __launch_bounds__(16 * TY, (sizeof(T) == 4 && TY == 16) ? 2 : 1)
-    inverse_kernel(T* Aall, int n, long long stride, int* flag) {
+    inverse_kernel(T* Aall, int n, long long stride, int* flag, const int* only) {
+  if (only && !only[blockIdx.x]) return;
   __shared__ T colk[2][INV_MAX_N];
   __shared__ T rowp[2][INV_MAX_N];
   __shared__ int perm[INV_MAX_N];   // perm[k] = pivot row of step k
@@ -690,7 +698,8 @@ __device__ __forceinline__ void warp_argmax(T best, int bi, int n, T& mbest, int
 
 template <typename T, int NW, int CW, int RL, int MB>
 __global__ void __launch_bounds__(32 * NW, MB)
-    inverse_wcol_kernel(T* Aall, int n, long long stride, int* flag) {
+    inverse_wcol_kernel(T* Aall, int n, long long stride, int* flag, InvMask mask) {
+  if (mask.only && !mask.only[blockIdx.x]) return;
   __shared__ T colb[2][32 * RL];
   __shared__ int sp[2];
   __shared__ T sd[2];
@@ -820,7 +829,7 @@ __global__ void __launch_bounds__(32 * NW, MB)
       }
     }
   }
-  if (singular && lane == 0) atomicExch(flag, 1);
+  if (singular && lane == 0) atomicExch(flag + mask.fs * blockIdx.x, 1);
   __syncthreads();
   for (int t = threadIdx.x; t < n; t += blockDim.x) pos[perm[t]] = t;
   __syncthreads();
@@ -841,15 +850,15 @@ constexpr int kInvVariants = 4;
 inline int inv_shape(int n, int v) { return (n <= 64 ? 4 : (n <= 96 ? 2 : 0)) + (v & 1); }
 
 template <typename T>
-int launch_wcol(int v, T* A, int n, long long stride, int batch, int* d_flag, cudaStream_t st) {
+int launch_wcol(int v, T* A, int n, long long stride, int batch, int* d_flag, cudaStream_t st, InvMask mask = {}) {
   constexpr bool F = sizeof(T) == 4;
   switch (inv_shape(n, v)) {
-    case 0: inverse_wcol_kernel<T, 8, 16, 4, F ? 2 : 1><<<batch, 256, 0, st>>>(A, n, stride, d_flag); break;
-    case 1: inverse_wcol_kernel<T, 16, 8, 4, F ? 2 : 1><<<batch, 512, 0, st>>>(A, n, stride, d_flag); break;
-    case 2: inverse_wcol_kernel<T, 6, 16, 3, F ? 3 : 2><<<batch, 192, 0, st>>>(A, n, stride, d_flag); break;
-    case 3: inverse_wcol_kernel<T, 12, 8, 3, F ? 2 : 1><<<batch, 384, 0, st>>>(A, n, stride, d_flag); break;
-    case 4: inverse_wcol_kernel<T, 4, 16, 2, F ? 6 : 4><<<batch, 128, 0, st>>>(A, n, stride, d_flag); break;
-    default: inverse_wcol_kernel<T, 8, 8, 2, F ? 4 : 3><<<batch, 256, 0, st>>>(A, n, stride, d_flag); break;
+    case 0: inverse_wcol_kernel<T, 8, 16, 4, F ? 2 : 1><<<batch, 256, 0, st>>>(A, n, stride, d_flag, mask); break;
+    case 1: inverse_wcol_kernel<T, 16, 8, 4, F ? 2 : 1><<<batch, 512, 0, st>>>(A, n, stride, d_flag, mask); break;
+    case 2: inverse_wcol_kernel<T, 6, 16, 3, F ? 3 : 2><<<batch, 192, 0, st>>>(A, n, stride, d_flag, mask); break;
+    case 3: inverse_wcol_kernel<T, 12, 8, 3, F ? 2 : 1><<<batch, 384, 0, st>>>(A, n, stride, d_flag, mask); break;
+    case 4: inverse_wcol_kernel<T, 4, 16, 2, F ? 6 : 4><<<batch, 128, 0, st>>>(A, n, stride, d_flag, mask); break;
+    default: inverse_wcol_kernel<T, 8, 8, 2, F ? 4 : 3><<<batch, 256, 0, st>>>(A, n, stride, d_flag, mask); break;
   }
   EXA_LAUNCH_CHECK();
   return EXA_OK;
@@ -872,15 +881,15 @@ int inv_variant(int n, bool fp64) {
 }
 
 template <typename T, int TY, int RR, int RC>
-int launch_inverse(T* A, int n, long long stride, int batch, int* d_flag, cudaStream_t st) {
+int launch_inverse(T* A, int n, long long stride, int batch, int* d_flag, cudaStream_t st, const int* only) {
   static_assert(TY * RR <= INV_MAX_N + 31 && 16 * RC <= INV_MAX_N, "inverse tile exceeds the buffers");
-  inverse_kernel<T, TY, RR, RC><<<batch, 16 * TY, 0, st>>>(A, n, stride, d_flag);
+  inverse_kernel<T, TY, RR, RC><<<batch, 16 * TY, 0, st>>>(A, n, stride, d_flag, only);
   EXA_LAUNCH_CHECK();
   return EXA_OK;
 }
 
 template <typename T>
-int inverse_dispatch(T* A, int n, long long stride, int batch, int* d_flag, cudaStream_t st) {
+int inverse_dispatch(T* A, int n, long long stride, int batch, int* d_flag, cudaStream_t st, InvMask mask = {}) {
   if (batch <= 0) return EXA_OK;
   if (n > INV_MAX_N || n <= 0) {
     exa_set_error("dense inverse of order %d exceeds the register kernel limit %d", n, INV_MAX_N);
@@ -901,13 +910,13 @@ int inverse_dispatch(T* A, int n, long long stride, int batch, int* d_flag, cuda
   }
   const int rc = (n + 15) / 16;
   // FP32 blocks up to 128: 256 threads with 8 x 8 entries each, two CTAs per SM
-  if (n <= 128) return launch_wcol<T>(inv_variant(n, sizeof(T) == 8), A, n, stride, batch, d_flag, st);
+  if (n <= 128) return launch_wcol<T>(inv_variant(n, sizeof(T) == 8), A, n, stride, batch, d_flag, st, mask);
   const int rr = (n + 31) / 32;
-  if (rr <= 2 && rc <= 4) return launch_inverse<T, 32, 2, 4>(A, n, stride, batch, d_flag, st);
-  if (rr <= 2 && rc <= 6) return launch_inverse<T, 32, 2, 6>(A, n, stride, batch, d_flag, st);
-  if (rr <= 3 && rc <= 6) return launch_inverse<T, 32, 3, 6>(A, n, stride, batch, d_flag, st);
-  if (rr <= 4 && rc <= 8) return launch_inverse<T, 32, 4, 8>(A, n, stride, batch, d_flag, st);
-  return launch_inverse<T, 32, 5, 10>(A, n, stride, batch, d_flag, st);
+  if (rr <= 2 && rc <= 4) return launch_inverse<T, 32, 2, 4>(A, n, stride, batch, d_flag, st, mask.only);
+  if (rr <= 2 && rc <= 6) return launch_inverse<T, 32, 2, 6>(A, n, stride, batch, d_flag, st, mask.only);
+  if (rr <= 3 && rc <= 6) return launch_inverse<T, 32, 3, 6>(A, n, stride, batch, d_flag, st, mask.only);
+  if (rr <= 4 && rc <= 8) return launch_inverse<T, 32, 4, 8>(A, n, stride, batch, d_flag, st, mask.only);
+  return launch_inverse<T, 32, 5, 10>(A, n, stride, batch, d_flag, st, mask.only);
 }
 }  // namespace
 
@@ -1000,7 +1009,7 @@ int exa_inverse_tune(int n, int batch, int fp64, cudaStream_t st) {
 //   X = A11^-1 (Gauss-Jordan, pivoting within the block), W1 = X A12, S = A22 - A21 W1,
 //   Y = S^-1, W3 = A21 X;  inverse = [X + W1 Y W3, -W1 Y; -Y W3, Y].
 // The products run on the FP64 DMMA GEMM (or an FP32 SIMT GEMM for the FP32 blocks).
-// Workspace: n^2 entries per matrix.
+// Workspace: n^2 + 1 entries per matrix.
 // ----------------------------------------------------------------------------------
 namespace {
 // C(r, c) = alpha sum_k A(r, k) B(k, c) + beta C(r, c), one batch entry per blockIdx.y;
@@ -1051,11 +1060,12 @@ __global__ void __launch_bounds__(256) simt_gemm_kernel(int M, int N, int K, T a
     }
 }
 
-// batched sub-matrix copy: dst(r, c) = src(r, c) for r < R, c < Cn
+// batched sub-matrix copy: dst(r, c) = src(r, c) for r < R, c < Cn (only: as InvMask's)
 template <typename T>
 __global__ void submat_copy_kernel(T* dst, long long ldd, long long sd, const T* src, long long lds, long long ss,
-                                   int R, int Cn) {
+                                   int R, int Cn, const int* only) {
   const long long b = blockIdx.y;
+  if (only && !only[b]) return;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < R * Cn; t += gridDim.x * blockDim.x) {
     const int r = t % R, c = t / R;
     dst[b * sd + r + ldd * c] = src[b * ss + r + lds * c];
@@ -1082,24 +1092,23 @@ int bgemm(int M, int N, int K, T alpha, T beta, const T* A, long long lda, long 
 
 template <typename T>
 int subcopy(T* dst, long long ldd, long long sd, const T* src, long long lds, long long ss, int R, int Cn, int batch,
-            cudaStream_t st) {
+            cudaStream_t st, const int* only = nullptr) {
   for (int b0 = 0; b0 < batch; b0 += 65535) {
     const int nb = (batch - b0 < 65535) ? batch - b0 : 65535;
     dim3 grid((unsigned)exa_ceil_div(R * Cn, 256 * 4), (unsigned)nb);
-    submat_copy_kernel<T><<<grid, 256, 0, st>>>(dst + b0 * sd, ldd, sd, src + b0 * ss, lds, ss, R, Cn);
+    submat_copy_kernel<T><<<grid, 256, 0, st>>>(dst + b0 * sd, ldd, sd, src + b0 * ss, lds, ss, R, Cn,
+                                                only ? only + b0 : nullptr);
     EXA_LAUNCH_CHECK();
   }
   return EXA_OK;
 }
 
-// The diagonal blocks are inverted the same way down to INV_LEAF (order 320: leaves of 80, whose
-// register kernel keeps several CTAs on an SM; one CTA per SM held a 160 x 160 leaf), in the part of
-// the workspace that is not in use yet.  1000 blocks of order 320 13.0 -> 9.8 ms (B200).  sw: entries
-// between matrices in the workspace.
-constexpr int INV_LEAF = 96;
-template <typename T>
-int inverse_blocked(T* A, int n, long long stride, int batch, T* ws, long long sw, int* d_flag, cudaStream_t st) {
-  if (n <= INV_LEAF) return inverse_dispatch<T>(A, n, stride, batch, d_flag, st);
+// The block formula in place on A, workspace n^2 entries per matrix, sw apart.  leaf(B, k, free, O) inverts
+// the order-k block B (spaced sw) in place, O being the same block where it still lies in A and `free`
+// workspace not in use, k^2 entries per matrix; before_y runs with S in A22 and Y = S^-1 in its argument.
+template <typename T, typename Leaf, typename BeforeY>
+int inverse_2x2(T* A, int n, long long stride, int batch, T* ws, long long sw, Leaf leaf, BeforeY before_y,
+                cudaStream_t st) {
   const int n1 = (n + 1) / 2, n2 = n - n1;
   T* W0 = ws;                                  // n1 x n1: A11, then X
   T* W1 = W0 + (long long)n1 * n1;             // n1 x n2: X A12
@@ -1110,18 +1119,116 @@ int inverse_blocked(T* A, int n, long long stride, int batch, T* ws, long long s
   T* A12 = A + (long long)n * n1;
   T* A22 = A + n1 + (long long)n * n1;
   EXA_TRY(subcopy<T>(W0, n1, sw, A11, n, stride, n1, n1, batch, st));
-  EXA_TRY(inverse_blocked<T>(W0, n1, sw, batch, W1, sw, d_flag, st));
+  EXA_TRY(leaf(W0, n1, W1, A11));
   EXA_TRY(bgemm<T>(n1, n2, n1, T(1), T(0), W0, n1, sw, A12, n, stride, W1, n1, sw, batch, st));
   EXA_TRY(bgemm<T>(n2, n2, n1, T(-1), T(1), A21, n, stride, W1, n1, sw, A22, n, stride, batch, st));
   EXA_TRY(subcopy<T>(W2, n2, sw, A22, n, stride, n2, n2, batch, st));
-  EXA_TRY(inverse_blocked<T>(W2, n2, sw, batch, W3, sw, d_flag, st));
+  EXA_TRY(leaf(W2, n2, W3, A22));
   EXA_TRY(bgemm<T>(n2, n1, n1, T(1), T(0), A21, n, stride, W0, n1, sw, W3, n2, sw, batch, st));
   EXA_TRY(bgemm<T>(n1, n2, n2, T(-1), T(0), W1, n1, sw, W2, n2, sw, A12, n, stride, batch, st));
   EXA_TRY(subcopy<T>(A11, n, stride, W0, n1, sw, n1, n1, batch, st));
   EXA_TRY(bgemm<T>(n1, n1, n2, T(-1), T(1), A12, n, stride, W3, n2, sw, A11, n, stride, batch, st));
   EXA_TRY(bgemm<T>(n2, n1, n2, T(-1), T(0), W2, n2, sw, W3, n2, sw, A21, n, stride, batch, st));
+  EXA_TRY(before_y(W0, W2));
   EXA_TRY(subcopy<T>(A22, n, stride, W2, n2, sw, n2, n2, batch, st));
   return EXA_OK;
+}
+
+// The halves are inverted by the same formula down to INV_LEAF (order 320: leaves of 80, whose
+// register kernel keeps several CTAs on an SM; one CTA per SM holds a 160 x 160 block).  1000 blocks of
+// order 320 13.0 -> 9.8 ms (B200).
+//
+// Pivots do not cross leaves, so a regular half whose own leading block is singular or nearly so would
+// be lost: the leading 80 rows of a 3D Euler block at p = 3 are the density nodes and one layer of
+// x momentum, singular without the time term.  The loss shows as growth: X = A11^-1 beside the half's
+// inverse, or S = A22 - A21 X A12 beside A22.  A half that grows by more than INV_GROWTH, or meets a
+// zero pivot or a non-finite entry, is inverted again from its original by the register kernel, which
+// pivots over all its rows.  Euler blocks (condition 380 to 2800, states perturbed by 1e-2): growth 1.0
+// at dtfactor 68, 1.4 at 1, with errors as from whole halves (2e-15); 6.9 at 0.1, where the leaves alone
+// lose a digit; 1e5 at 1e-6, where they leave two digits.
+constexpr int INV_LEAF = 96;
+constexpr double INV_GROWTH = 2.0;
+
+// redo[b] = 1 where the half's inverse [A; A22 still S, its inverse in Y] is not to be kept.  O22: A22 of
+// the original half, leading dimension ldo, so apart.  One CTA per matrix.
+template <typename T>
+__global__ void __launch_bounds__(256) inverse_growth_kernel(int n, int n1, const T* A, long long stride, const T* X,
+                                                             const T* Y, long long sw, const T* O22, long long ldo,
+                                                             long long so, int* redo) {
+  const long long b = blockIdx.x;
+  const int n2 = n - n1, tid = threadIdx.x;
+  A += b * stride;
+  X += b * sw;
+  Y += b * sw;
+  O22 += b * so;
+  const T big = sizeof(T) == 8 ? T(1.7976931348623157e308) : T(3.4028235e38f);
+  T m[4] = {T(0), T(0), T(0), T(0)};  // the inverse, X, S, A22
+  bool bad = false;
+  auto take = [&](int k, T v) {
+    v = absval(v);
+    if (!(v <= big)) bad = true;  // infinities and NaN
+    else if (v > m[k]) m[k] = v;
+  };
+  for (int t = tid; t < n * n; t += 256) {
+    const int r = t % n, c = t / n;
+    take(r >= n1 && c >= n1 ? 2 : 0, A[t]);
+  }
+  for (int t = tid; t < n1 * n1; t += 256) take(1, X[t]);
+  for (int t = tid; t < n2 * n2; t += 256) {
+    take(0, Y[t]);
+    take(3, O22[t % n2 + ldo * (t / n2)]);
+  }
+  __shared__ T red[8][4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+      const T o = __shfl_xor_sync(0xffffffffu, m[k], off);
+      m[k] = o > m[k] ? o : m[k];
+    }
+    if ((tid & 31) == 0) red[tid >> 5][k] = m[k];
+  }
+  bad = __syncthreads_or(bad);
+  if (tid != 0) return;
+#pragma unroll
+  for (int q = 1; q < 8; ++q)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) m[k] = red[q][k] > m[k] ? red[q][k] : m[k];
+  if (bad || m[1] > T(INV_GROWTH) * m[0] || m[2] > T(INV_GROWTH) * m[3]) redo[b] = 1;
+}
+
+// The inverse of a half of order up to INV_MAX_N, spaced sw, in place.  O: the half where it lies
+// unchanged; redo: one int per matrix.
+template <typename T>
+int inverse_half(T* A, int n, int batch, T* ws, long long sw, const T* O, long long ldo, long long so, int* redo,
+                 int* d_flag, cudaStream_t st) {
+  if (n <= INV_LEAF) return inverse_dispatch<T>(A, n, sw, batch, d_flag, st);
+  EXA_CUDA(cudaMemsetAsync(redo, 0, sizeof(int) * (size_t)batch, st));
+  const int n1 = (n + 1) / 2;
+  EXA_TRY(inverse_2x2<T>(
+      A, n, sw, batch, ws, sw,
+      [&](T* B, int k, T*, const T*) { return inverse_dispatch<T>(B, k, sw, batch, redo, st, InvMask{nullptr, 1}); },
+      [&](const T* X, const T* Y) -> int {
+        inverse_growth_kernel<T><<<batch, 256, 0, st>>>(n, n1, A, sw, X, Y, sw, O + n1 + ldo * n1, ldo, so, redo);
+        EXA_LAUNCH_CHECK();
+        return EXA_OK;
+      },
+      st));
+  EXA_TRY(subcopy<T>(A, n, sw, O, ldo, so, n, n, batch, st, redo));
+  return inverse_dispatch<T>(A, n, sw, batch, d_flag, st, InvMask{redo, 0});
+}
+
+// ws: n^2 entries per matrix, then one int per matrix
+template <typename T>
+int inverse_blocked(T* A, int n, long long stride, int batch, T* ws, int* d_flag, cudaStream_t st) {
+  const long long sw = (long long)n * n;
+  int* redo = reinterpret_cast<int*>(ws + sw * batch);
+  return inverse_2x2<T>(
+      A, n, stride, batch, ws, sw,
+      [&](T* B, int k, T* free, const T* O) {
+        return inverse_half<T>(B, k, batch, free, sw, O, n, stride, redo, d_flag, st);
+      },
+      [](const T*, const T*) { return EXA_OK; }, st);
 }
 
 template <typename T>
@@ -1132,10 +1239,10 @@ int inverse_ws(T* A, int n, long long stride, int batch, T* ws, int* d_flag, cud
     return EXA_ERR_UNSUPPORTED;
   }
   if (!ws) {
-    exa_set_error("dense inverse of order %d needs a workspace of n^2 entries per matrix", n);
+    exa_set_error("dense inverse of order %d needs a workspace of n^2 + 1 entries per matrix", n);
     return EXA_ERR_ARG;
   }
-  return inverse_blocked<T>(A, n, stride, batch, ws, (long long)n * n, d_flag, st);
+  return inverse_blocked<T>(A, n, stride, batch, ws, d_flag, st);
 }
 }  // namespace
 
@@ -1277,7 +1384,7 @@ int exa_inverse_tc32(float* A, int n, long long stride, int batch, float* ws, fl
 }
 
 int exa_inverse_max_n() { return 2 * INV_MAX_N; }
-int exa_inverse_needs_ws(int n) { return n > INV_MAX_N; }
+size_t exa_inverse_ws_size(int n) { return n > INV_MAX_N ? (size_t)n * n + 1 : 0; }
 
 int exa_inverse_ws(double* A, int n, long long stride, int batch, double* ws, int* d_flag, cudaStream_t st) {
   return inverse_ws<double>(A, n, stride, batch, ws, d_flag, st);

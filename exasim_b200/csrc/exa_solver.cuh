@@ -70,7 +70,7 @@ struct ExaCtx {
   int wT_elems = 0;
   bool k_given = false;    // a caller holds or has written the "K" field: its zeros are set again
   int* face_k = nullptr;   // without q: the element unknowns on each face [npf ncu, nfe], increasing
-  double* wInv = nullptr;  // blocked-inverse workspace (n^2 per element) when n exceeds the register kernel
+  double* wInv = nullptr;  // blocked-inverse workspace when n exceeds the register kernel
   // Krylov / Newton workspace
   double *V = nullptr, *x = nullptr, *r = nullptr, *w = nullptr, *we = nullptr, *du = nullptr;
   double *part_a = nullptr, *part_b = nullptr, *part_m = nullptr, *hess = nullptr, *gs = nullptr, *gcs = nullptr,

@@ -155,3 +155,88 @@ def test_every_tuned_shape_gives_the_same_bits(lib, fp64):
         assert np.abs(got - ref).max() / np.abs(ref).max() < tol
     v = ctypes.c_int(-2)
     assert lib.exa_inverse_autotune(200, fp64, 8, None, ctypes.byref(v)) == 0 and v.value == -1
+
+
+@pytest.mark.parametrize("n", [193, 200, 250, 319, 320])
+@pytest.mark.parametrize("lead", ["zero", "tiny", "regular"])
+def test_pivots_are_found_beyond_the_leaves(lib, n, lead):
+    """Blocks whose leading quarter is singular (or scaled by 1e-9) while their leading half is regular and
+    well conditioned: the halves are [[e R, Q], [Q', R']] with orthogonal Q, in both diagonal places.  Without
+    pivots from outside the quarter the scaled one loses nine digits and the singular one everything; every
+    other matrix of the batch is an ordinary one, and must not be affected.  The blocks have cond 5: pivoting
+    over the halves leaves 2e-14 in a 64-bit restatement of the steps (leaves of 96 rows: 1e-6 and NaN);
+    1e-12 as above."""
+    import torch
+    rng = np.random.default_rng(n)
+    batch = 12
+    h, q = (n + 1) // 2, ((n + 1) // 2 + 1) // 2
+    eps = {"zero": 0.0, "tiny": 1e-9, "regular": 1.0}[lead]
+    orth = lambda k: np.linalg.qr(rng.standard_normal((k, k)))[0]
+
+    def half(k, lead_rows):
+        M = 0.1 * rng.standard_normal((k, k)) / np.sqrt(k)
+        r = k - lead_rows
+        M[:lead_rows, :lead_rows] = eps * orth(lead_rows)
+        M[:r, lead_rows:] += orth(r)
+        M[lead_rows:, :r] += orth(r)
+        if lead_rows > r:  # one more leading row than there are others: it needs an entry of its own
+            M[r, r] = 1.0
+        return M
+
+    A = 0.02 * rng.standard_normal((batch, n, n)) / np.sqrt(n)
+    for b in range(batch):
+        if b % 2 == 0:
+            A[b, :h, :h] = half(h, q)
+            A[b, h:, h:] = half(n - h, (n - h + 1) // 2)
+        else:
+            A[b] += rng.standard_normal((n, n)) + np.eye(n) * (2.0 * np.sqrt(n))
+    assert np.linalg.cond(A).max() < 10
+    ref = np.linalg.inv(A)
+    dev = torch.tensor(np.ascontiguousarray(np.transpose(A, (0, 2, 1))).ravel(), dtype=torch.float64, device="cuda")
+    flag = torch.zeros(1, dtype=torch.int32, device="cuda")
+    st = lib.exa_dinverse_batched(ctypes.c_void_p(dev.data_ptr()), n, n * n, batch, ctypes.c_void_p(flag.data_ptr()),
+                                  None)
+    assert st == 0, lib.exa_last_error().decode()
+    torch.cuda.synchronize()
+    got = np.transpose(dev.cpu().numpy().reshape(batch, n, n), (0, 2, 1))
+    err = np.abs(got - ref).max((1, 2)) / np.abs(ref).max((1, 2))
+    print(n, lead, f"{err.max():.1e}")
+    assert int(flag.item()) == 0
+    assert err.max() < 1e-12
+    # a singular block sets the flag at these orders too
+    A[0] = 0.0
+    dev = torch.tensor(np.ascontiguousarray(np.transpose(A, (0, 2, 1))).ravel(), dtype=torch.float64, device="cuda")
+    assert lib.exa_dinverse_batched(ctypes.c_void_p(dev.data_ptr()), n, n * n, batch, ctypes.c_void_p(flag.data_ptr()),
+                                    None) == 0
+    torch.cuda.synchronize()
+    assert int(flag.item()) == 1
+
+
+@pytest.mark.parametrize("dtfactor", [45.0, 0.1, 1e-6, 0.0])
+def test_euler_blocks_with_a_weak_time_term(tmp_path, dtfactor):
+    """The p = 3 blocks of 3D Euler, whose leading 80 rows (density and one layer of x momentum) become
+    singular as the time term goes: D^-1, D^-1 F and H against the oracle's LAPACK.  cond(D) is 2.8e3; pivoting
+    within 160 rows, as the kernel promises, leaves 1e-12 of D^-1 in 64-bit numpy (leaves of 80 rows: 1e-2 at
+    1e-6), times 1e2 for the products: 1e-10."""
+    from exasim_b200 import HDGSolver, cases
+    from oracle.hdg import HDGOracle
+    from oracle.models import MODELS
+    B.build(["euler3d"])
+    d = str(tmp_path / "datain")
+    cases.euler3d_vortex_hex(d, n=3, porder=3)
+    s, o = HDGSolver(d, "euler3d"), HDGOracle(d, MODELS["euler3d"]())
+    rng = np.random.default_rng(0)
+    o.udg = o.udg * (1 + 1e-2 * rng.standard_normal(o.udg.shape))
+    o.time, o.dtfactor = 0.01, dtfactor
+    o.sdg = dtfactor * o.udg[:, :o.ncu]
+    o.sdgg = np.einsum("gj,jce->gec", o.shapegt[:, :, 0], o.sdg)
+    s.set("udg", o.udg)
+    s.set("sdg", o.sdg)
+    s.set_time(o.time, o.dtfactor)
+    s.hdgAssembleLinearSystem()
+    H, Rh, F, Ru = o.assemble()
+    err = lambda a, b: np.abs(a - np.asarray(b).ravel(order="F")).max() / np.abs(b).max()
+    e = {k: err(s.get(k), v) for k, v in (("Dinv", o.Dinv), ("F", F), ("H", H), ("Ru", Ru), ("Rh", Rh))}
+    s.close()
+    print(dtfactor, {k: f"{v:.1e}" for k, v in e.items()})
+    assert max(e.values()) < 1e-10
