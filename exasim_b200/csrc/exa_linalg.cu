@@ -352,11 +352,11 @@ int exa_gemm(const GemmBatch& g, cudaStream_t st) {
     }
     return EXA_OK;
   }
-  if (g.kidx && (g.K > 512 || g.N == 1)) {
-    exa_set_error("gemm over a list of k: K = %d, N = %d", g.K, g.N);
+  if (g.kidx && g.K > 512) {
+    exa_set_error("gemm over a list of k: K = %d", g.K);
     return EXA_ERR_ARG;
   }
-  if (g.N == 1) {
+  if (g.N == 1 && !g.kidx) {  // a list of k goes with one column too: faces of one unknown
     dim3 grid((unsigned)exa_ceil_div(g.M, 128), (unsigned)g.batch, (unsigned)g.batch2);
     gemv_batch_kernel<<<grid, 128, 0, st>>>(g);
     EXA_LAUNCH_CHECK();
