@@ -1021,12 +1021,12 @@ int exa_get_field(exa_ctx* h, const char* name, double* host, long long n) {
 int exa_set_field(exa_ctx* h, const char* name, const double* host, long long n) {
   EXA_TRY(guard(h));
   FieldRef f{};
-  if (name && std::string(name) == "K") h->c.k_given = true;
   if (!field(h->c, name, f) || !host || n != f.n) {
     exa_set_error("set_field('%s'): unknown name or size %lld != %lld", name ? name : "", n, f.n);
     return EXA_ERR_ARG;
   }
   if (f.p == h->c.wB) h->c.b_pending = false;
+  if (f.p && f.p == h->c.wK) h->c.k_given = true;
   EXA_CUDA(cudaStreamSynchronize(h->c.st));
   if (n && f.p32) {
     std::vector<float> t(host, host + n);
@@ -1040,11 +1040,11 @@ int exa_set_field(exa_ctx* h, const char* name, const double* host, long long n)
 int exa_field_ptr(exa_ctx* h, const char* name, double** dev, long long* n) {
   EXA_TRY(guard(h));
   FieldRef f{};
-  if (name && std::string(name) == "K") h->c.k_given = true;
   if (!field(h->c, name, f) || !dev || !n) {
     exa_set_error("field_ptr('%s'): unknown name", name ? name : "");
     return EXA_ERR_ARG;
   }
+  if (f.p && f.p == h->c.wK) h->c.k_given = true;
   if (f.p == h->c.wB) {  // the pointer shows B of every later assembly too
     EXA_TRY(exa_model_form_b(h->c));
     h->c.b_given = true;

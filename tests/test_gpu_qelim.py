@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 import torch
 
-from exasim_b200 import HDGSolver, build as B, cases
+from exasim_b200 import ExaError, HDGSolver, build as B, cases
 from oracle.hdg import HDGOracle
 from oracle.models import MODELS
 
@@ -84,6 +84,39 @@ def test_blocks_without_q_are_assembled_again(tmp_path, n, p):
         for name, ref in (("H", H), ("F", F), ("Ru", Ru), ("Rh", Rh)):
             assert err(s.get(name), ref) < 5e-12, name
     assert err(s.get("K"), o.K) < 1e-11
+    s.close()
+
+
+def test_refused_calls_for_k_change_nothing(tmp_path):
+    """Once a caller holds or has written K, each assembly sets its zeros again (two more memory sets per
+    chunk); a call for it that is refused does not count."""
+    from torch.profiler import ProfilerActivity, profile
+    B.build(["euler3d"])
+    d = str(tmp_path / "datain")
+    cases.euler3d_vortex_hex(d, n=2, porder=2, periodic=False)
+    s = HDGSolver(d, "euler3d")
+    s.set_time(0.01, 45.0)
+    s.set("sdg", 45.0 * s.get("udg"))
+
+    def sets():
+        s.hdgAssembleLinearSystem()
+        torch.cuda.synchronize()
+        with profile(activities=[ProfilerActivity.CUDA]) as prof:
+            s.hdgAssembleLinearSystem()
+            torch.cuda.synchronize()
+        names = [e.name for e in prof.events()]
+        assert any("face_kernel" in n for n in names), names
+        return sum(n.startswith("Memset (") for n in names)
+
+    before = sets()
+    for call in (lambda: s.set("K", np.zeros(3)), lambda: s.lib.exa_field_ptr(s.h, b"K", None, None)):
+        try:
+            assert call() not in (None, 0)
+        except ExaError:
+            pass
+        assert sets() == before
+    s.set("K", s.get("K"))
+    assert sets() == before + 2
     s.close()
 
 
