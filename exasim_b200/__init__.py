@@ -51,6 +51,7 @@ def load_library(model: str) -> ctypes.CDLL:
         "exa_sizes": ([P, PLL], I),
         "exa_get_field": ([P, ctypes.c_char_p, P, LL], I),
         "exa_set_field": ([P, ctypes.c_char_p, P, LL], I),
+        "exa_field_size": ([P, ctypes.c_char_p, PLL], I),
         "exa_field_ptr": ([P, ctypes.c_char_p, ctypes.POINTER(P), PLL], I),
         "exa_get_connectivity": ([P, P, P], I),
         "exa_set_time": ([P, D, D], I),
@@ -146,8 +147,8 @@ class HDGSolver:
 
     # ---- data access
     def field_size(self, name: str) -> int:
-        p, n = ctypes.c_void_p(), ctypes.c_longlong()
-        self._check(self.lib.exa_field_ptr(self.h, name.encode(), ctypes.byref(p), ctypes.byref(n)))
+        n = ctypes.c_longlong()
+        self._check(self.lib.exa_field_size(self.h, name.encode(), ctypes.byref(n)))
         return int(n.value)
 
     def field_ptr(self, name: str):

@@ -1037,6 +1037,17 @@ int exa_set_field(exa_ctx* h, const char* name, const double* host, long long n)
   return EXA_OK;
 }
 
+int exa_field_size(exa_ctx* h, const char* name, long long* n) {
+  EXA_TRY(guard(h));
+  FieldRef f{};
+  if (!field(h->c, name, f) || !n) {
+    exa_set_error("field_size('%s'): unknown name", name ? name : "");
+    return EXA_ERR_ARG;
+  }
+  *n = f.n;
+  return EXA_OK;
+}
+
 int exa_field_ptr(exa_ctx* h, const char* name, double** dev, long long* n) {
   EXA_TRY(guard(h));
   FieldRef f{};

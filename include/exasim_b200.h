@@ -59,7 +59,10 @@ int exa_sizes(exa_ctx* ctx, long long* out);
  * and exa_field_ptr returns their device address (pointing at floats). */
 int exa_get_field(exa_ctx* ctx, const char* name, double* host, long long n);
 int exa_set_field(exa_ctx* ctx, const char* name, const double* host, long long n);
-/* Device pointer and length of a named array (zero-copy access, e.g. from torch). */
+/* Length of a named array. */
+int exa_field_size(exa_ctx* ctx, const char* name, long long* n);
+/* Device pointer and length of a named array (zero-copy access, e.g. from torch).  A caller that holds
+ * "K" or "B" sees every later assembly's, which then sets K's zeros and forms B each time. */
 int exa_field_ptr(exa_ctx* ctx, const char* name, double** dev, long long* n);
 /* f2e [4, nf] and elemcon [npf*nfe, ne] (0-based), either may be NULL. */
 int exa_get_connectivity(exa_ctx* ctx, int* f2e, int* elemcon);

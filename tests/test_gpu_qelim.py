@@ -87,6 +87,31 @@ def test_blocks_without_q_are_assembled_again(tmp_path, n, p):
     s.close()
 
 
+def test_reading_a_block_does_not_form_it_for_good(tmp_path):
+    """get() of B forms B once (two launches) and leaves the later assemblies as they were; a pointer to it
+    makes each of them form it."""
+    B.build(["convdiff3d"])
+    d = str(tmp_path / "datain")
+    cases.convdiff3d_hex(d, n=2, porder=3)
+    s = HDGSolver(d, "convdiff3d")
+    s.set_time(0.01, 45.0)
+
+    def launches(call):
+        before = s.lib.exa_launch_count()
+        call()
+        return s.lib.exa_launch_count() - before
+
+    s.hdgAssembleLinearSystem()
+    first = launches(s.hdgAssembleLinearSystem)
+    assert s.field_size("B") == s.sizes["n"] * 3 * s.sizes["n"] * s.sizes["ne"]
+    b = []
+    assert launches(lambda: b.append(s.get("B"))) == 2 and np.abs(b[0]).max() > 0
+    assert launches(s.hdgAssembleLinearSystem) == first
+    s.field_ptr("B")
+    assert launches(s.hdgAssembleLinearSystem) == first + 2
+    s.close()
+
+
 def test_refused_calls_for_k_change_nothing(tmp_path):
     """Once a caller holds or has written K, each assembly sets its zeros again (two more memory sets per
     chunk); a call for it that is refused does not count."""
