@@ -152,7 +152,9 @@ int schur_chunk(ExaCtx& c, int e0, int nb) {
     EXA_TRY(exa_inverse_ws(c.wD, n, (long long)n * n, nb, c.wInv, c.d_flag, c.st));
   }
   ExaProfScope ps(c, EXA_PH_SCHUR);
-  exa_prof_flops(c, EXA_PH_SCHUR, 2.0 * nb * ((double)n * n * m + (double)n * n + (double)m * m * n + (double)m * n));
+  // D^-1 F and K D^-1 F run over the k that face_k lists, a face's unknowns, where it does
+  const double kf = c.face_k ? (double)P.npf * ncu : (double)n;
+  exa_prof_flops(c, EXA_PH_SCHUR, 2.0 * nb * ((double)n * m * kf + (double)n * n + (double)m * m * kf + (double)m * n));
   GemmBatch g{};
   g.batch = nb; g.batch2 = 1;
   // DinvF = -Dinv F.  Without q the columns of F on face l have entries at that face's nodes only,

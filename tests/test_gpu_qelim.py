@@ -112,6 +112,29 @@ def test_reading_a_block_does_not_form_it_for_good(tmp_path):
     s.close()
 
 
+@pytest.mark.parametrize("model,p", [("euler3d", 2), ("convdiff3d", 2)])
+def test_schur_products_are_counted_as_they_run(tmp_path, model, p):
+    """The products of the Schur phase: D^-1 F and K D^-1 F with all n rows, or (without q) those of a face."""
+    B.build([model])
+    d = str(tmp_path / "datain")
+    if model == "euler3d":
+        cases.euler3d_vortex_hex(d, n=2, porder=p, periodic=False)
+    else:
+        cases.convdiff3d_hex(d, n=2, porder=p)
+    s = HDGSolver(d, model)
+    s.set_time(0.01, 45.0)
+    s.set("sdg", 45.0 * s.get("udg")[:s.sizes["n"] * s.sizes["ne"]])
+    s.hdgAssembleLinearSystem()
+    s.profile(True)
+    s.hdgAssembleLinearSystem()
+    z, flops = s.sizes, s.profile_read()["schur"][2]
+    s.profile(False)
+    n, m, ne = z["n"], z["m"], z["ne"]
+    k = z["npf"] * z["ncu"] if model == "euler3d" else n
+    assert flops == 2.0 * ne * (n * m * k + n * n + m * m * k + m * n)
+    s.close()
+
+
 def test_refused_calls_for_k_change_nothing(tmp_path):
     """Once a caller holds or has written K, each assembly sets its zeros again (two more memory sets per
     chunk); a call for it that is refused does not count."""
