@@ -125,7 +125,12 @@ void find_tensor(ExaTensor& t, const Blob& M, const ExaDims& P, int elemtype) {
   for (int g = 0; g < n1; ++g) t.w[g] = M.part[21][g];
   // tables [rows, cols, 1 + dims]: to the points (g, a) and, weighted, back (a, g)
   auto matches = [&](const double* T, const double* W, int dims, int n) {
-    double big = 0.0, off = 0.0;
+    double big = 0.0;
+    for (long long k = 0; k < (long long)n * n * (dims + 1); ++k) big = std::max(big, std::fabs(T[k]));
+    // The solver then uses the products in place of the file's tables, so results move by what those are
+    // off, times the cancellation in the derivatives: at 1e-14 of the largest entry, by 1e-12 to 1e-11.  Tables
+    // from the inverse of the nodes' Vandermonde matrix are off by 1e-16 to 2e-15 (orders 1 to 5).
+    const double tol = 1e-14 * big;
     for (int d = 0; d <= dims; ++d)
       for (int a = 0; a < n; ++a)
         for (int g = 0; g < n; ++g) {
@@ -135,10 +140,9 @@ void find_tensor(ExaTensor& t, const Blob& M, const ExaDims& P, int elemtype) {
             w *= t.w[ga % n1];
           }
           const double tv = T[g + (size_t)n * (a + (size_t)n * d)], wv = W[a + (size_t)n * (g + (size_t)n * d)];
-          big = std::max(big, std::fabs(tv));
-          off = std::max(off, std::max(std::fabs(tv - v), std::fabs(wv - v * w)));
+          if (!(std::fabs(tv - v) <= tol) || !(std::fabs(wv - v * w) <= tol)) return false;
         }
-    return off <= 1e-13 * big;
+    return true;
   };
   if (matches(M.part[1], M.part[2], P.nd, np) && matches(M.part[3], M.part[4], P.nd - 1, nf)) t.n1 = n1;
 }

@@ -62,3 +62,40 @@ def test_residual_and_blocks_match_oracle(tmp_path, model, n, p):
     print(model, n, p, {k: f"{v:.1e}" for k, v in e.items()})
     assert e["udg"] < 1e-11 and e["Ru"] < 1e-11 and e["Rh"] < 1e-11
     assert max(e["H"], e["F"]) < (2e-11 if p == 4 else 5e-12)
+
+
+@pytest.mark.parametrize("off", [3e-14, 1e-9])
+def test_tables_that_are_no_products_are_used_as_they_are(tmp_path, off):
+    """A master file whose element tables differ from the Kronecker products of its 1D ones by more than
+    rounding: q and the residual are those of the file's tables (sums of 1e3 terms in another order: 2e-12 of
+    the largest entry), not of the products, which 3e-14 would put ten times as far off."""
+    from exasim_b200 import inputs as I
+    B.build(["convdiff3d"])
+    d = str(tmp_path / "datain")
+    cases.convdiff3d_hex(d, n=2, porder=4, nsteps=1)
+    m = I.make_master(3, 1, 4, 8)
+    rng = np.random.default_rng(5)
+    shap = m.shapegt + off * np.abs(m.shapegt).max() * rng.uniform(-1, 1, m.shapegt.shape)
+    m.shapegt, m.shapegw = I._shapes_t_w(np.transpose(shap, (1, 0, 2)), m.gwe, 4)
+    I.write_master_bin(d + "/master.bin", m)
+    s, o = HDGSolver(d, "convdiff3d"), HDGOracle(d, MODELS["convdiff3d"]())
+    udg, uh = rng.standard_normal(o.udg.shape), rng.standard_normal(o.uh.shape)
+    o.udg, o.uh = udg.copy(), uh.copy()
+    o.time, o.dtfactor = 0.01, 45.0
+    o.sdg = 40.0 * udg[:, :1]
+    o.sdgg = np.einsum("gj,jce->gec", o.shapegt[:, :, 0], o.sdg)
+    s.set("udg", udg)
+    s.set("uh", uh)
+    s.set("sdg", o.sdg)
+    s.set_time(o.time, o.dtfactor)
+    s.hdgGetQ()
+    o.get_q(o.udg, o.uh)
+    err = lambda a, b: np.abs(a - np.asarray(b).ravel(order="F")).max() / np.abs(b).max()
+    e = {"udg": err(s.get("udg"), o.udg)}
+    s.set("udg", o.udg)
+    s.hdgAssembleResidual()
+    Ru, Rh = o.residual()[:2]
+    e["Ru"], e["Rh"] = err(s.get("Ru"), Ru), err(s.get("Rh"), Rh)
+    s.close()
+    print(off, {k: f"{v:.1e}" for k, v in e.items()})
+    assert max(e.values()) < 2e-12
