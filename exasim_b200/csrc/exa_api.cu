@@ -112,15 +112,19 @@ int init_solution(ExaCtx& c, const Blob& S) {
 
 // The 1D tables of the master element when its shape tables are their Kronecker products to
 // rounding (quadrilaterals and hexahedra with as many Gauss points as nodes per dimension); the
-// file's own 1D tables (parts shap1dgt and gw1d) are checked against every table used.
-void find_tensor(ExaTensor& t, const Blob& M, const ExaDims& P, int elemtype) {
+// file's own 1D tables (parts shap1dgt and gw1d) are checked against every table used.  slots:
+// the face nodes (a + npf l) that each element node is, in order, -1 beyond the last [nd, npe].
+void find_tensor(ExaTensor& t, std::vector<int>& slots, const Blob& M, const ExaDims& P, int elemtype,
+                 const std::vector<int>& perm) {
   t.n1 = 0;
   if (elemtype != 1 || P.nd < 2 || P.nd > 3 || M.nsize.size() < 22) return;
   int n1 = 1;
   while ((P.nd == 3 ? n1 * n1 * n1 : n1 * n1) < P.npe) ++n1;
   const int np = P.nd == 3 ? n1 * n1 * n1 : n1 * n1, nf = np / n1;
   if (n1 > EXA_TP_MAX || np != P.npe || P.nge != np || P.npf != nf || P.ngf != nf) return;
-  if (M.nsize[15] != 2LL * n1 * n1 || M.nsize[21] != n1) return;
+  if (M.nsize[15] != 2LL * n1 * n1 || M.nsize[21] != n1 || (int)perm.size() != P.ndf) return;
+  for (int k = 1; k <= 4; ++k)
+    if (M.nsize[k] != (k <= 2 ? (long long)np * np * (P.nd + 1) : (long long)nf * nf * P.nd)) return;
   for (int q = 0; q < n1 * n1; ++q) t.S[q] = M.part[15][q], t.D[q] = M.part[15][n1 * n1 + q];
   for (int g = 0; g < n1; ++g) t.w[g] = M.part[21][g];
   // tables [rows, cols, 1 + dims]: to the points (g, a) and, weighted, back (a, g)
@@ -144,7 +148,17 @@ void find_tensor(ExaTensor& t, const Blob& M, const ExaDims& P, int elemtype) {
         }
     return true;
   };
-  if (matches(M.part[1], M.part[2], P.nd, np) && matches(M.part[3], M.part[4], P.nd - 1, nf)) t.n1 = n1;
+  if (!matches(M.part[1], M.part[2], P.nd, np) || !matches(M.part[3], M.part[4], P.nd - 1, nf)) return;
+  slots.assign((size_t)P.nd * P.npe, -1);
+  for (int s = 0; s < P.ndf; ++s) {
+    if (perm[s] < 0 || perm[s] >= P.npe) return;
+    int* q = &slots[(size_t)P.nd * perm[s]];
+    int k = 0;
+    while (k < P.nd && q[k] >= 0) ++k;
+    if (k == P.nd) return;  // a node on more faces than the element has dimensions
+    q[k] = s;
+  }
+  t.n1 = n1;
 }
 
 int exa_ctx_init(ExaCtx& c, const double* app, long long napp, const double* master, long long nmaster,
@@ -373,19 +387,9 @@ int exa_ctx_init(ExaCtx& c, const double* app, long long napp, const double* mas
   EXA_TRY(dev_alloc(c, &c.elemg, ne * P.elemg_stride()));
   EXA_TRY(dev_alloc(c, &c.faceg, ne * P.nfe * P.faceg_stride()));
   EXA_TRY(exa_k_geometry(P, c.shapegt, c.shapfgt, c.perm, c.xdg, c.elemg, c.faceg, c.st));
-  find_tensor(c.tensor, M, P, c.elemtype);
-  if (c.tensor.n1 > 0) {
-    std::vector<int> ns((size_t)P.nd * P.npe, -1);
-    bool ok = true;
-    for (int t = 0; t < P.ndf && ok; ++t) {
-      int* q = &ns[(size_t)P.nd * perm[t]];
-      int k = 0;
-      while (k < P.nd && q[k] >= 0) ++k;
-      ok = k < P.nd;
-      if (ok) q[k] = t;
-    }
-    if (ok) EXA_TRY(dev_upload(c, &c.tp_nslot, ns.data(), ns.size()));
-  }
+  std::vector<int> slots;
+  find_tensor(c.tensor, slots, M, P, c.elemtype, perm);
+  if (c.tensor.n1 > 0) EXA_TRY(dev_upload(c, &c.tp_nslot, slots.data(), slots.size()));
   if (c.scheme == 0) {
     // LDG: both sides' face-node table, the face nodal basis for the boundary's Ubou, and
     // the residual buffers of the finite-difference Jacobian
@@ -438,14 +442,16 @@ int exa_ctx_init(ExaCtx& c, const double* app, long long napp, const double* mas
     EXA_TRY(exa_inverse_tune(P.npe, (int)std::min<size_t>(ne, 4096), 1, c.st));
     EXA_TRY(exa_inverse(mass, P.npe, (long long)P.npe * P.npe, P.ne, c.d_flag, c.st));
     c.Minv = mass;  // kept: q recovery applies it to C u - E uhat
-    EXA_TRY(dev_alloc(c, &c.wq_ug, ne * P.nge * P.ncu));
-    EXA_TRY(dev_alloc(c, &c.wq_v, ne * P.nge * P.nd * P.nd * P.ncu));
-    EXA_TRY(dev_alloc(c, &c.wq_w, ne * P.npe * P.nd * P.ncu));
-    // the two products of q recovery over all elements: u at the Gauss points (one batch entry
-    // per field) and the gradient moments C_d u (large meshes only, as above)
-    if ((long long)ne * P.nge * P.npe >= (1LL << 25)) {
-      EXA_TRY(exa_gemm_tune(P.nge, (int)ne, P.npe, P.ncu, c.st));
-      EXA_TRY(exa_gemm_tune(P.npe, P.ncu * P.nd * (int)ne, P.nge * P.nd, 1, c.st));
+    if (!exa_model_has_getq_tp(P, c.tensor)) {
+      EXA_TRY(dev_alloc(c, &c.wq_ug, ne * P.nge * P.ncu));
+      EXA_TRY(dev_alloc(c, &c.wq_v, ne * P.nge * P.nd * P.nd * P.ncu));
+      EXA_TRY(dev_alloc(c, &c.wq_w, ne * P.npe * P.nd * P.ncu));
+      // the two products of q recovery over all elements: u at the Gauss points (one batch entry
+      // per field) and the gradient moments C_d u (large meshes only, as above)
+      if ((long long)ne * P.nge * P.npe >= (1LL << 25)) {
+        EXA_TRY(exa_gemm_tune(P.nge, (int)ne, P.npe, P.ncu, c.st));
+        EXA_TRY(exa_gemm_tune(P.npe, P.ncu * P.nd * (int)ne, P.nge * P.nd, 1, c.st));
+      }
     }
     GemmBatch g{};
     g.M = P.npe; g.N = P.npe; g.K = P.npe; g.alpha = 1.0; g.beta = 0.0;
@@ -504,7 +510,11 @@ int exa_ctx_init(ExaCtx& c, const double* app, long long napp, const double* mas
   // element chunk: bounded workspace (about 8 GB at most)
   const size_t inv_ws = hdg ? exa_inverse_ws_size((int)n) : 0;
   const size_t vol_ws = (size_t)P.nge * P.nc + (size_t)P.nge * P.ncu + (size_t)P.nge * (P.nd + 1) * P.ncu;
-  const size_t per_elem = hdg ? sizeof(double) * (n * n + n * nqn + n * m + m * n + m * nqn +
+  // with the q elimination by sum factorization neither B nor G is formed, but the face fluxes'
+  // derivatives with respect to q are kept (B is made when a caller asks for it: block_b)
+  const bool qtp = hdg && exa_model_qelim_tp(P, c.tensor);
+  const size_t bg = qtp ? 2 * (size_t)P.nfe * P.ngf * P.ncu * P.ncq : (n + m) * nqn;
+  const size_t per_elem = hdg ? sizeof(double) * (n * n + n * m + m * n + bg +
                                                   (size_t)P.nge * (P.nd + 1) * P.ncu * P.nc + n + inv_ws)
                               : sizeof(double) * (vol_ws + n);
   size_t cap = (size_t)8 << 30;
@@ -512,13 +522,16 @@ int exa_ctx_init(ExaCtx& c, const double* app, long long napp, const double* mas
   const size_t nb = c.neb;
   if (hdg) {
     EXA_TRY(dev_alloc(c, &c.wD, nb * n * n));
-    EXA_TRY(dev_alloc(c, &c.wB, std::max<size_t>(1, nb * n * nqn)));
     EXA_TRY(dev_alloc(c, &c.wF, nb * n * m));
     EXA_TRY(dev_alloc(c, &c.wK, nb * m * n));
-    EXA_TRY(dev_alloc(c, &c.wG, std::max<size_t>(1, nb * m * nqn)));
+    if (qtp) {
+      EXA_TRY(dev_alloc(c, &c.wFq, nb * bg));
+    } else {
+      EXA_TRY(dev_alloc(c, &c.wB, std::max<size_t>(1, nb * n * nqn)));
+      EXA_TRY(dev_alloc(c, &c.wG, std::max<size_t>(1, nb * m * nqn)));
+    }
     EXA_TRY(dev_alloc(c, &c.wRg, nb * P.nge * (P.nd + 1) * P.ncu * P.nc));
     EXA_TRY(dev_alloc(c, &c.wRu, nb * n));
-    if (exa_model_qelim_tp(c)) EXA_TRY(dev_alloc(c, &c.wFq, nb * 2 * P.nfe * P.ngf * P.ncu * P.ncq));
   }
   EXA_TRY(dev_alloc(c, &c.wUG, nb * P.nge * P.nc));
   EXA_TRY(dev_alloc(c, &c.wSG, nb * P.nge * P.ncu));
@@ -553,7 +566,7 @@ int exa_ctx_init(ExaCtx& c, const double* app, long long napp, const double* mas
     // the FP64 element products of the assembly: the fastest GEMM tile of each shape is
     // measured once per process and device (q elimination, D^-1 F, K D^-1 F)
     const int kq = P.npe * P.nd, nbt = (int)std::min<size_t>(nb, 512);
-    if (P.ncq > 0) {
+    if (P.ncq > 0 && !qtp) {
       EXA_TRY(exa_gemm_tune((int)n, P.npe, kq, nbt, c.st));
       EXA_TRY(exa_gemm_tune((int)n, P.ndf, kq, nbt, c.st));
       EXA_TRY(exa_gemm_tune((int)m, P.npe, kq, nbt, c.st));
@@ -742,7 +755,7 @@ int exa_ctx_set_precision(ExaCtx& c, int mode) {
       EXA_TRY(exa_pack(c.ME, 1, kq, 1, (long long)kq * P.ndf, 0, (int)ne, 1, c.MEp, c.st, kg, P.npe));
       // B and G as A operands, one part per trace component b, with the same K
       EXA_TRY(packed(c.wBp, P.n, kq4, 128, nb, P.ncu, false));
-      EXA_TRY(packed(c.wGp, P.m, kq4, 128, nb, P.ncu, false));
+      if (!c.wFq) EXA_TRY(packed(c.wGp, P.m, kq4, 128, nb, P.ncu, false));
     }
     if (exa_vol_mat_tc_fits(P)) {
       // basis at the Gauss points: row j (node), k = g
@@ -836,35 +849,70 @@ unsigned long long exa_ctx_key(const double* app, long long napp, const double* 
   return h;
 }
 
-// Device bytes a context for these blobs will hold (the arrays exa_ctx_init allocates, with
-// nf bounded by ne * nfe), for admission before it exists; 0 for malformed blobs.
+// Device bytes a context for these blobs will hold at most (the arrays exa_ctx_init and
+// exa_ctx_set_precision allocate, with nf bounded by ne * nfe), for admission before it exists; 0 for
+// malformed blobs.
 long long exa_ctx_estimate_bytes(const double* app, long long napp, const double* master, long long nmaster,
                                  const double* mesh, long long nmesh, int precision) {
   Blob A = split_blob(app, napp), M = split_blob(master, nmaster), Me = split_blob(mesh, nmesh);
-  if (!A.ok || !M.ok || !Me.ok || A.nsize.size() < 9 || M.nsize.size() < 1 || Me.nsize.size() < 1) return 0;
-  const double ncu = A.part[0][6], nc = A.part[0][5], ncq = A.part[0][7];
-  const double restart = A.part[2][15], precond = A.part[1][6];
-  const double nd = M.part[0][0], npe = M.part[0][5], npf = M.part[0][6], nge = M.part[0][7], ngf = M.part[0][8];
-  const double ne = Me.part[0][1], nfe = Me.part[0][4];
-  const double nf = ne * nfe, n = npe * ncu, ndf = npf * nfe, m = ndf * ncu, N = ncu * npf * nf;
-  const double nqn = ncq > 0 ? npe * nd * ncu : 0;
-  double per_elem = m * m + n * m + n + m + npe * nc + npe * ncu + nge * (nd + nd * nd + 1) + nfe * ngf * (2 * nd + 1) +
-                    (ncq > 0 ? npe * npe * nd + npe * ndf * nd + npe * npe * (2 + nd) + npe * ndf * nd : 0) + m + n;
-  // q recovery workspace (Gauss-point u, its geometric products, C u)
-  per_elem += ncq > 0 ? nge * ncu * (1 + nd * nd) + npe * nd * ncu : 0;
-  per_elem += precond == 1 ? m * m : 0;
-  // element chunk workspace (the whole mesh when it fits in 8 GB)
-  per_elem += n * n + n * nqn + 2 * n * m + m * nqn + nge * (nd + 1) * ncu * nc + n + (n > 160 ? n * n : 0);
-  per_elem += nge * (nc + ncu + (nd + 1) * ncu);  // Gauss-point values and Ru integrand of a chunk
+  if (!A.ok || !M.ok || !Me.ok || A.nsize.size() < 9 || M.nsize.size() < 1 || Me.nsize.size() < 1 ||
+      A.nsize[0] < 12 || A.nsize[1] < 7 || A.nsize[2] < 17 || M.nsize[0] < 9 || Me.nsize[0] < 5)
+    return 0;
+  ExaDims P{};
+  P.ncu = (int)A.part[0][6], P.nc = (int)A.part[0][5], P.ncq = (int)A.part[0][7], P.ncx = (int)A.part[0][11];
+  P.nd = (int)M.part[0][0], P.npe = (int)M.part[0][5], P.npf = (int)M.part[0][6], P.nge = (int)M.part[0][7];
+  P.ngf = (int)M.part[0][8], P.ne = (int)Me.part[0][1], P.nfe = (int)Me.part[0][4];
+  if (P.ncu < 1 || P.nc < 1 || P.nd < 1 || P.npe < 1 || P.npf < 1 || P.nge < 1 || P.ngf < 1 || P.ne < 1 || P.nfe < 1)
+    return 0;
+  P.ndf = P.npf * P.nfe;
+  P.n = P.npe * P.ncu;
+  P.m = P.ncu * P.ndf;
+  ExaTensor t;
+  std::vector<int> slots;
+  if (Me.nsize.size() > 23)
+    find_tensor(t, slots, M, P, (int)M.part[0][1], to_int(Me.part[23], Me.nsize[23]));
+  const bool hdg = A.part[2][0] != 0.0;
+  const int precond = (int)A.part[1][6];
+  const double restart = A.part[2][15], rbdim = A.part[2][16], poly = A.nsize[2] > 27 ? A.part[2][27] : 0.0;
+  const double ne = P.ne, nd = P.nd, npe = P.npe, ndf = P.ndf, ncu = P.ncu, nc = P.nc, nge = P.nge, n = P.n, m = P.m;
+  const double nf = ne * P.nfe, ncf = ncu * P.npf, N = std::max(ncf * nf, hdg ? 0.0 : n * ne);
+  const bool q = P.ncq > 0, qtp = hdg && exa_model_qelim_tp(P, t);
+  const double rg = nge * (nd + 1) * ncu * nc, ug = nge * (nc + ncu + (nd + 1) * ncu);
+  const double bg = qtp ? 2.0 * P.nfe * P.ngf * ncu * P.ncq : (q ? (n + m) * npe * nd * ncu : 0.0);
+  const double inv = hdg ? (double)exa_inverse_ws_size(P.n) : 0.0;
+  // as exa_ctx_init: the element chunk
+  const double per = hdg ? n * n + 2 * n * m + bg + rg + n + inv : ug + n;
+  const double nb = std::max(1.0, std::min(std::min(ne, std::floor((8LL << 30) / (8.0 * per))), 65535.0));
   // preconditioner blocks: block Jacobi one per face; block ILU(0) one per stored block of the
   // sub-domain face graph, at most the face itself and the other faces of its two elements
-  const double ncf2 = ncu * npf * ncu * npf;
-  const double pblocks = precond == 0 ? ncf2 * nf : (precond == 2 ? ncf2 * nf * (1 + 2 * (nfe - 1)) : 0.0);
+  const double pblocks = precond == 0 ? ncf * ncf * nf : (precond == 2 ? ncf * ncf * nf * (1 + 2 * (P.nfe - 1)) : ne * m * m);
+  double words = ne * (npe * (nd + nc + ncu) + P.elemg_stride() + P.nfe * P.faceg_stride() + 2 * n + ndf);
+  words += N * (restart + 6) + ncf * nf + nf * 4 + 1e5;
+  if (poly > 1) words += 3 * N;
+  words += 2 * N * rbdim;
+  if (A.part[1][0] != 0.0) words += 2 * ne * n;
+  if (q) words += ne * (npe * npe * (1 + 2 * nd) + 2 * npe * ndf * nd);
+  if (q && !exa_model_has_getq_tp(P, t)) words += ne * (nge * ncu * (1 + nd * nd) + npe * nd * ncu);
+  words += nb * ug;
+  if (!hdg) {
+    words += 4 * ne * n + ncf * nf * 2 + ne * npe * npe;
+    return (long long)(8.0 * words) + (16LL << 20);
+  }
+  words += ne * 2 * m + nb * (n * n + 2 * n * m + bg + rg + n + inv);
   // volume-product T factors: at most 512 MB
-  const double wt = std::min(ne * npe * nge * ncu * nc, (double)(64 << 20));
-  double words = ne * per_elem + N * (restart + 6) + pblocks + wt;
-  if (precision == 1) words *= 1.75;
-  return (long long)(8.0 * words) + (16LL << 20);
+  if (!exa_tensor_blocks(P, t)) words += std::min(nb * npe * nge * ncu * nc, (double)(64 << 20));
+  const double full = ne * (m * m + n * m) + pblocks;  // H, D^-1 F and the preconditioner in FP64
+  double most = words + full;
+  if (precision == 1) {
+    // these are freed but for one chunk of H, and the FP32 arrays come instead
+    const int kq = exa_tc::qk_group(P.npe) * P.nd;
+    double f = ne * (m * m + 2 * n * m + n * n) + pblocks;
+    if (q) f += ne * (exa_pack_size(P.npe, kq) + exa_pack_size(P.ndf, kq)) + nb * ncu * exa_pack_size(P.n, kq);
+    if (q && !qtp) f += nb * ncu * exa_pack_size(P.m, kq);
+    f += nb * (exa_pack_size(P.n, P.n) + 3 * exa_pack_size(P.m, P.n) + exa_inverse_tc32_ws(P.n) + exa_inverse_tc32_pk(P.n));
+    most = std::max(most, words + nb * m * m + 0.5 * f + nge * npe * (nd + 4));
+  }
+  return (long long)(8.0 * most) + (16LL << 20);
 }
 
 void exa_ctx_free(ExaCtx& c) {
@@ -911,7 +959,16 @@ struct FieldRef {
   double* p;
   long long n;
   float* p32 = nullptr;  // FP32 arrays of the mixed-precision form (p is null then)
+  bool b = false;        // "B", which is allocated and formed on request where the solver does without
 };
+
+int block_b(ExaCtx& c, FieldRef& f, bool form) {
+  if (!c.wB) EXA_TRY(dev_alloc(c, &c.wB, (size_t)f.n));
+  f.p = c.wB;
+  if (form) return exa_model_form_b(c);
+  c.b_pending = false;
+  return EXA_OK;
+}
 
 bool field(ExaCtx& c, const char* name, FieldRef& f) {
   const ExaDims& P = c.P;
@@ -940,8 +997,10 @@ bool field(ExaCtx& c, const char* name, FieldRef& f) {
   else if (s == "elemg") f = {c.elemg, (long long)P.elemg_stride() * ne};
   else if (s == "faceg") f = {c.faceg, (long long)P.faceg_stride() * P.nfe * ne};
   else if (s == "K" && c.neb == P.ne) f = {c.wK, m * n * ne};
-  else if (s == "B" && c.neb == P.ne && !(c.precision == 1 && c.Sp.hi))  // else B exists only packed in FP32
+  else if (s == "B" && c.neb == P.ne && !(c.precision == 1 && c.Sp.hi)) {  // else B exists only packed in FP32
     f = {c.wB, n * (long long)P.npe * P.nd * P.ncu * ne};
+    f.b = true;
+  }
   else if (s == "Dinv" && c.neb == P.ne) f = {c.wD, n * n * ne};
   else if (s == "H32" && c.H32) f = {nullptr, m * m * ne, c.H32};
   else if (s == "F32" && c.F32) f = {nullptr, n * m * ne, c.F32};
@@ -1010,7 +1069,7 @@ int exa_get_field(exa_ctx* h, const char* name, double* host, long long n) {
     exa_set_error("get_field('%s'): unknown name or size %lld != %lld", name ? name : "", n, f.n);
     return EXA_ERR_ARG;
   }
-  if (f.p == h->c.wB) EXA_TRY(exa_model_form_b(h->c));
+  if (f.b) EXA_TRY(block_b(h->c, f, true));
   EXA_CUDA(cudaStreamSynchronize(h->c.st));
   if (n && f.p32) {
     std::vector<float> t((size_t)n);
@@ -1029,7 +1088,7 @@ int exa_set_field(exa_ctx* h, const char* name, const double* host, long long n)
     exa_set_error("set_field('%s'): unknown name or size %lld != %lld", name ? name : "", n, f.n);
     return EXA_ERR_ARG;
   }
-  if (f.p == h->c.wB) h->c.b_pending = false;
+  if (f.b) EXA_TRY(block_b(h->c, f, false));
   if (f.p && f.p == h->c.wK) h->c.k_given = true;
   EXA_CUDA(cudaStreamSynchronize(h->c.st));
   if (n && f.p32) {
@@ -1060,8 +1119,8 @@ int exa_field_ptr(exa_ctx* h, const char* name, double** dev, long long* n) {
     return EXA_ERR_ARG;
   }
   if (f.p && f.p == h->c.wK) h->c.k_given = true;
-  if (f.p == h->c.wB) {  // the pointer shows B of every later assembly too
-    EXA_TRY(exa_model_form_b(h->c));
+  if (f.b) {  // the pointer shows B of every later assembly too
+    EXA_TRY(block_b(h->c, f, true));
     h->c.b_given = true;
   }
   *dev = f.p32 ? reinterpret_cast<double*>(f.p32) : f.p;

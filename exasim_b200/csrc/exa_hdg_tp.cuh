@@ -450,6 +450,11 @@ bool launch_hdg_resid_tp(const AsmArgs& A, const ExaTensor& T, const int* nslot,
   return false;
 }
 
+// the pairs and orders of launch_getq_tp
+inline bool getq_tp_fits(const ExaDims& P, const ExaTensor& T) {
+  const bool pair = P.nd == 2 ? P.ncu == 1 || P.ncu == 4 : P.nd == 3 && P.ncu == 1;
+  return pair && P.nfe == 2 * P.nd && T.n1 >= 3 && T.n1 <= 5;
+}
 inline bool launch_getq_tp(const ExaDims& P, const ExaTensor& T, const int* nslot, const int* perm, const int* elemcon,
                            const double* elemg, const double* faceg, const double* uh, double* udg, cudaStream_t st,
                            int* rc) {

@@ -526,14 +526,17 @@ bool exa_model_getq_tp(ExaCtx& c, int* rc) {
   return c.tp_nslot && launch_getq_tp(c.P, c.tensor, c.tp_nslot, c.perm, c.elemcon, c.elemg, c.faceg, c.uh, c.udg, c.st, rc);
 }
 
-bool exa_model_qelim_tp(const ExaCtx& c) {
-  return c.tp_nslot && exa_tensor_blocks(c.P, c.tensor) && qelim_tp_fits(c.P, c.tensor);
+bool exa_model_has_getq_tp(const ExaDims& P, const ExaTensor& t) { return P.ncq > 0 && getq_tp_fits(P, t); }
+
+// the mixed form's volume kernel then packs B itself, so neither form stores B and G
+bool exa_model_qelim_tp(const ExaDims& P, const ExaTensor& t) {
+  return exa_tensor_blocks(P, t) && qelim_tp_fits(P, t) && exa_vol_mat_tc_fits(P);
 }
 
 int exa_model_form_b(ExaCtx& c) {
   const ExaDims& P = c.P;
   int rc = EXA_OK;
-  if (!c.b_pending) return EXA_OK;
+  if (!c.b_pending || !c.wB) return EXA_OK;
   c.b_pending = false;
   if (!launch_vol_blocks_tp(P, c.tensor, c.wRg, c.wD, c.wB, P.ncu, P.nc, P.ne, c.st, &rc))
     return EXA_OK;

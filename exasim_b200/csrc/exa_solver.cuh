@@ -53,13 +53,16 @@ struct ExaCtx {
   double *udg = nullptr, *uh = nullptr, *sdg = nullptr;
   double *MC = nullptr, *ME = nullptr;
   double* Minv = nullptr;  // inverse element mass matrices [npe, npe, ne] (q recovery by quadrature)
-  // q recovery workspace: Gauss-point u, its geometric products and C_d u for all elements
+  // q recovery workspace: Gauss-point u, its geometric products and C_d u for all elements (null where
+  // the tensor-product kernel recovers q)
   double *wq_ug = nullptr, *wq_v = nullptr, *wq_w = nullptr;
   double *H = nullptr, *F = nullptr, *Ru = nullptr, *Rh = nullptr, *b = nullptr, *Pc = nullptr;
   // assembly workspace for a chunk of `neb` elements
   int neb = 0;
   double *wD = nullptr, *wB = nullptr, *wF = nullptr, *wK = nullptr, *wG = nullptr, *wRg = nullptr, *wRu = nullptr;
-  double* wFq = nullptr;  // derivatives of the face fluxes with respect to q (tensor-product q elimination), per chunk
+  // derivatives of the face fluxes with respect to q (tensor-product q elimination), per chunk; with it
+  // there is no wG, and wB only once a caller has asked for B
+  double* wFq = nullptr;
   bool b_pending = false;  // B of the last assembly is not formed yet (exa_model_form_b)
   bool b_given = false;    // a caller holds the "B" pointer: every assembly forms it
   // per chunk: udg and sdg at the Gauss points and the Ru integrand (the volume kernel's GEMMs)
@@ -179,9 +182,10 @@ int exa_model_assemble(ExaCtx& c, bool jacobian);
 int exa_model_init_udg(ExaCtx& c, double* host_udg);
 // q recovery of tensor-product elements; false where there is no instance (*rc: its status)
 bool exa_model_getq_tp(ExaCtx& c, int* rc);
+bool exa_model_has_getq_tp(const ExaDims& P, const ExaTensor& t);
 // whether the q elimination applies B and G by sum factorization (wFq) instead of forming them, and
 // B of the last assembly for callers that read the field
-bool exa_model_qelim_tp(const ExaCtx& c);
+bool exa_model_qelim_tp(const ExaDims& P, const ExaTensor& t);
 int exa_model_form_b(ExaCtx& c);
 // LDG residual (residual.cpp:589-617) of the element states u [npe, ncu, ne] into Ru
 int exa_model_ldg_residual(ExaCtx& c, const double* u, double* Ru);
