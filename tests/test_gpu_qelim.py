@@ -168,7 +168,7 @@ def test_refused_calls_for_k_change_nothing(tmp_path):
     s.close()
 
 
-@pytest.mark.parametrize("n,p", [(2, 2), (3, 3), (2, 4), (3, 4)])
+@pytest.mark.parametrize("n,p", [(2, 2), (3, 3), (2, 4), (3, 4), (5, 2)])
 def test_mixed_blocks_match_oracle(tmp_path, n, p):
     """K and H of the mixed form, whose trace rows are eliminated face by face in FP32 (rounding 6e-8 of
     sums that cancel to a tenth: 5e-6), H behind a D^-1 of condition 1e3 (2e-4)."""
