@@ -795,9 +795,10 @@ def run_served(args, device):
 # blocks are read once).
 QELIM_TRAFFIC_PER_ELEMENT = 2.326e9 / 1331
 # The same for the mixed form's q elimination: two 3xTF32 products (umma3_kernel, FP32 operands
-# split on chip), 0.564 and 0.642 GB read + written on the 10^3 mesh, and the trace rows
-# (trace_q_kernel), 0.534 GB on the 9^3 mesh.
-QELIM_MIXED_TRAFFIC_PER_ELEMENT = (0.564e9 + 0.642e9) / 1000 + 0.534e9 / 729
+# split on chip), 0.564 and 0.642 GB read + written on the 10^3 mesh (the mean per launch), and the
+# trace rows (trace_q_kernel), 0.534 GB on the 9^3 mesh.
+QELIM_MIXED_TRAFFIC_PER_ELEMENT_LAUNCH = (0.564e9 + 0.642e9) / 1000 / 2
+TRACE_ROWS_TRAFFIC_PER_ELEMENT = 0.534e9 / 729
 
 
 def fp64_gemm_peak(torch):
@@ -833,41 +834,44 @@ def qelim_mixed_bytes(sz):
     and packed (the A operand of K D^-1 F)."""
     npe, nd, ne, ncu = sz["npe"], sz["nd"], sz["ne"], sz.get("ncu", 1)
     ndf = sz["npf"] * sz["nfe"]
-    n, m, kq = npe * ncu, ndf * ncu, npe * nd
-    d = 4 * ncu * n * kq + 4 * kq * npe + 8 * n * npe * ncu + 4 * n * npe * ncu
-    f = 4 * ncu * n * kq + 4 * kq * ndf + 8 * n * ndf * ncu + 4 * n * ndf * ncu
+    m, kq = ndf * ncu, npe * nd
     k = 4 * ncu * m * kq + 4 * kq * npe + 8 * m * npe * ncu + 8 * m * npe * ncu
     h = 4 * ncu * m * kq + 4 * kq * ndf + 8 * m * ndf * ncu + 4 * m * ndf * ncu
-    return (d + f + k + h) * ne
+    return qelim_products_bytes(sz) + (k + h) * ne
 
 
-def qelim_bytes(sz):
-    """The same without G, as scalar models on hexahedra run: the products D and F as above; the
-    trace rows read MinvC and MinvE, the FP64 flux derivatives and the face blocks of K and H, and
-    write K plain and packed and H plain."""
+def qelim_products_bytes(sz):
+    """The first two of them, D and F: the products that scalar models on hexahedra run."""
+    npe, nd, ne, ncu = sz["npe"], sz["nd"], sz["ne"], sz.get("ncu", 1)
+    ndf = sz["npf"] * sz["nfe"]
+    n, kq = npe * ncu, npe * nd
+    d = 4 * ncu * n * kq + 4 * kq * npe + 8 * n * npe * ncu + 4 * n * npe * ncu
+    f = 4 * ncu * n * kq + 4 * kq * ndf + 8 * n * ndf * ncu + 4 * n * ndf * ncu
+    return (d + f) * ne
+
+
+def trace_rows_bytes(sz):
+    """K and H there, without G: MinvC and MinvE, the FP64 flux derivatives and the face blocks of K
+    and H read, K plain and packed and H plain written."""
     npe, nd, ne = sz["npe"], sz["nd"], sz["ne"]
     ndf = sz["npf"] * sz["nfe"]
-    kq = npe * nd
-    df = 2 * 4 * npe * kq + 4 * kq * (npe + ndf) + 12 * npe * (npe + ndf)
-    trace = 4 * kq * (npe + ndf) + 8 * ndf * nd + 2 * 8 * ndf * sz["npf"] + 8 * ndf * npe + 4 * ndf * ndf
-    return (df + trace) * ne
+    return (4 * npe * nd * (npe + ndf) + 8 * ndf * nd + 2 * 8 * ndf * sz["npf"] + 8 * ndf * npe + 4 * ndf * ndf) * ne
 
 
 def autotuned(s):
     """The shapes the project's autotuners chose for this workload (timed on scratch blocks
     when the contexts were created): the element inverse of order n in FP32 and FP64 (shape
-    0-3 of the column-by-warp Gauss-Jordan) and the FP64 DMMA tile of each q-elimination and
-    Schur product (exa_dgemm_tune's index into its tiles)."""
+    0-3 of the column-by-warp Gauss-Jordan) and the FP64 DMMA tile of each Schur product
+    (exa_dgemm_tune's index into its tiles)."""
     import ctypes
     L, sz = s.lib, s.sizes
-    n, m, npe, ndf, nd = sz["n"], sz["m"], sz["npe"], sz["npf"] * sz["nfe"], sz["nd"]
+    n, m = sz["n"], sz["m"]
     out = {}
     for fp64 in (0, 1):
         v = ctypes.c_int(-1)
         L.exa_inverse_autotune(n, fp64, sz["ne"], None, ctypes.byref(v))
         out[f"inverse_n{n}_{'fp64' if fp64 else 'fp32'}_shape"] = v.value
-    for M, N, K in ((n, npe, npe * nd), (n, ndf, npe * nd), (m, npe, npe * nd), (m, ndf, npe * nd), (n, m, n),
-                    (m, m, n)):
+    for M, N, K in ((n, m, n), (m, m, n)):
         t = ctypes.c_int(-1)
         L.exa_dgemm_tune(M, N, K, min(sz["ne"], 512), None, ctypes.byref(t))
         out[f"dgemm_{M}x{N}x{K}_tile"] = t.value
@@ -875,28 +879,31 @@ def autotuned(s):
 
 
 def kernel_rooflines(s32, s64, mixed, plain, torch, steps):
-    """roofline: the q elimination of the mixed solve, two products of umma3_kernel on the TF32
-    tensor cores and trace_q_kernel, HBM-bound, from the phase timers (CUDA events on the solver's
-    stream around each q-elimination region) of the profiled solves that follow the timed ones.
-    The plain form's FP64 q elimination (qelim3_kernel) is reported beside it against cuBLAS
-    DGEMM, and the FP32 condensed matvec is timed alone on the solver's stream."""
+    """roofline: the two q-elimination products of the mixed solve, umma3_kernel on the TF32 tensor
+    cores, HBM-bound, from the phase timers (CUDA events on the solver's stream around each
+    q-elimination region, less the trace rows within it) of the profiled solves that follow the
+    timed ones; trace_roofline: those trace rows, trace_q_kernel.  The plain form's FP64 q
+    elimination (qelim3_kernel) is reported beside them against cuBLAS DGEMM, and the FP32 condensed
+    matvec is timed alone on the solver's stream."""
     peaks, src = measured_peaks()
     sz = s32.sizes
     ne, m, N = sz["ne"], sz["m"], sz["ndofuhat"]
     q_ms, q_regions, _ = mixed["prof"]["qelim"]
-    launches = 3 * q_regions
-    qbytes = qelim_bytes(sz)
-    ms_launch = q_ms / max(launches, 1)
-    achieved = qbytes / 3 / (ms_launch * 1e-3) / 1e9 if q_ms > 0 else 0.0
-    roofline = {"kernel": "umma3_kernel (q-elimination GEMMs D += B MinvC, F -= B MinvE; 3xTF32 on tcgen05: FP32 "
-                          "operands by cp.async.bulk, split into TF32 hi and lo parts in shared memory) and "
-                          "trace_q_kernel (K += G MinvC, H -= G MinvE by sum factorization in FP32)",
-                "bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
-                "frac": achieved / peaks["hbm_gbs"], "peak_source": src,
-                "algorithmic_bytes_per_launch": qbytes / 3, "dense_products_bytes": qelim_mixed_bytes(sz), "ms_per_launch": ms_launch, "launches": launches,
-                "traffic": QELIM_MIXED_TRAFFIC_PER_ELEMENT / 3 * ne,
-                "traffic_source": "ncu dram bytes of the three launches on smaller meshes, mean per launch, scaled by "
-                                  "element count"}
+    t_ms, t_regions, _ = mixed["prof"]["qelim_trace"]
+
+    def hbm(kernel, ms, launches, nbytes, traffic, mesh):
+        ms_launch = ms / max(launches, 1)
+        achieved = nbytes / (ms_launch * 1e-3) / 1e9 if ms > 0 else 0.0
+        return {"kernel": kernel, "bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
+                "frac": achieved / peaks["hbm_gbs"], "peak_source": src, "algorithmic_bytes_per_launch": nbytes,
+                "ms_per_launch": ms_launch, "launches": launches, "traffic": traffic * ne,
+                "traffic_source": f"ncu dram bytes of the same launches on {mesh} mesh, scaled by element count"}
+
+    roofline = hbm("umma3_kernel (q-elimination GEMMs D += B MinvC, F -= B MinvE; 3xTF32 on tcgen05: FP32 operands by "
+                   "cp.async.bulk, split into TF32 hi and lo parts in shared memory)", q_ms - t_ms, 2 * q_regions,
+                   qelim_products_bytes(sz) / 2, QELIM_MIXED_TRAFFIC_PER_ELEMENT_LAUNCH, "a 10^3")
+    trace = hbm("trace_q_kernel (K += G MinvC, H -= G MinvE by sum factorization in FP32)", t_ms, t_regions,
+                trace_rows_bytes(sz), TRACE_ROWS_TRAFFIC_PER_ELEMENT, "a 9^3")
     p_ms, p_regions, p_flops = plain["prof"]["qelim"]
     peak64 = fp64_gemm_peak(torch)
     pl = p_regions
@@ -931,7 +938,7 @@ def kernel_rooflines(s32, s64, mixed, plain, torch, steps):
                 "peak_source": src, "algorithmic_bytes_per_launch": nbytes, "ms_per_launch": ms}
 
     plain_roof["matvec_roofline"] = matvec_roof(s64, plain["stream"], 8, "FP64")
-    return {"roofline": roofline, "plain_roofline": plain_roof,
+    return {"roofline": roofline, "trace_roofline": trace, "plain_roofline": plain_roof,
             "matvec_roofline": matvec_roof(s32, mixed["stream"], 4, "FP32")}
 
 

@@ -269,9 +269,11 @@ int schur_chunk_mixed(ExaCtx& c, int e0, int nb) {
     u.out[0] = toF; u.nout = 1;
     EXA_TRY(exa_gemm_3xtf32(u, c.d_uflag, c.st));
     // K and H: G is applied from the flux derivatives where the elements are tensor products
-    if (tp_trace(c))
+    if (tp_trace(c)) {
+      ExaProfScope pt(c, EXA_PH_QTRACE);
       EXA_TRY(launch_trace_q(P, c.tensor, c.tp_nslot, c.perm, c.wFq, at(c.MCp, e0), at(c.MEp, e0), c.wK, Hc, K32, H32,
                              c.Kp, nb, c.st));
+    }
     // K(:, j + npe*b) = K + G_b MinvC, plain and packed (A operand of K D^-1 F)
     u.M = m; u.N = npe; u.alpha = 1.0;
     u.A = c.wGp; u.B = at(c.MCp, e0); u.B.sb2 = 0;

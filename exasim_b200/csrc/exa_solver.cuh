@@ -17,6 +17,7 @@
 enum ExaPhase {
   EXA_PH_VOLUME = 0, EXA_PH_FACE, EXA_PH_QELIM, EXA_PH_INVERSE, EXA_PH_SCHUR, EXA_PH_PRECOND_BUILD,
   EXA_PH_MATVEC, EXA_PH_PRECOND_APPLY, EXA_PH_ORTHO, EXA_PH_GETQ, EXA_PH_RESIDUAL, EXA_PH_PACK, EXA_PH_UPDATE,
+  EXA_PH_QTRACE,  // part of EXA_PH_QELIM: trace_q_kernel
   EXA_NPHASE
 };
 

@@ -34,6 +34,15 @@ def test_qelim_bytes_of_the_benchmark_assembly():
     assert per_elem == d + f + k + h == 2632500
 
 
+def test_qelim_bytes_by_kernel():
+    """What scalar models on hexahedra run: the products into D and F, and the trace rows without G."""
+    z = sizes()
+    df = 4 * (125 * 375 + 375 * 125) + 12 * 125 * 125 + 4 * (125 * 375 + 375 * 150) + 12 * 125 * 150
+    assert bench.qelim_products_bytes(z) == df * 16 ** 3
+    trace = 4 * 375 * 275 + 8 * 150 * 3 + 16 * 150 * 25 + 8 * 150 * 125 + 4 * 150 * 150
+    assert bench.trace_rows_bytes(z) == trace * 16 ** 3
+
+
 def test_phase_table_per_solve():
     prof = {"qelim": (36.0, 40, 4.0e12), "matvec": (19.5, 420, 0.0), "getq": (0.0, 0, 0.0)}
     out = bench.phases_of(prof, 10)

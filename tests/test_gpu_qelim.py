@@ -135,6 +135,24 @@ def test_schur_products_are_counted_as_they_run(tmp_path, model, p):
     s.close()
 
 
+def test_trace_rows_are_timed_within_the_q_elimination(tmp_path):
+    """Phase qelim_trace of the profile: one region per mixed assembly, within those of qelim; none in FP64."""
+    B.build(["convdiff3d"])
+    d = str(tmp_path / "datain")
+    cases.convdiff3d_hex(d, n=3, porder=4)
+    s = HDGSolver(d, "convdiff3d")
+    s.set_time(0.01, 45.0)
+    for mixed in (0, 1):
+        s.set_precision(mixed)
+        s.profile(True)
+        s.hdgAssembleLinearSystem()
+        p = s.profile_read()
+        s.profile(False)
+        assert p["qelim"][1] == 1 and p["qelim_trace"][1] == mixed
+        assert 0.0 <= p["qelim_trace"][0] < p["qelim"][0]
+    s.close()
+
+
 def test_refused_calls_for_k_change_nothing(tmp_path):
     """Once a caller holds or has written K, each assembly sets its zeros again (two more memory sets per
     chunk); a call for it that is refused does not count."""
