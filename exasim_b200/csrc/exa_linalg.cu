@@ -868,7 +868,7 @@ std::mutex g_inv_mu;
 std::map<std::array<int, 3>, int> g_inv_tune;  // (device, n, fp64) -> measured fastest variant
 
 // the measured variant for this order and type (2, 3: the shapes for orders up to 64), else the
-// default: FP32 16 columns per warp, FP64 8
+// default: FP32 16 columns per warp, FP64 8 (16 for orders 65 to 96)
 int inv_variant(int n, bool fp64) {
   int dev = 0;
   if (cudaGetDevice(&dev) == cudaSuccess) {
@@ -909,7 +909,6 @@ int inverse_dispatch(T* A, int n, long long stride, int batch, int* d_flag, cuda
     return EXA_OK;
   }
   const int rc = (n + 15) / 16;
-  // FP32 blocks up to 128: 256 threads with 8 x 8 entries each, two CTAs per SM
   if (n <= 128) return launch_wcol<T>(inv_variant(n, sizeof(T) == 8), A, n, stride, batch, d_flag, st, mask);
   const int rr = (n + 31) / 32;
   if (rr <= 2 && rc <= 4) return launch_inverse<T, 32, 2, 4>(A, n, stride, batch, d_flag, st, mask.only);
@@ -1095,7 +1094,7 @@ int subcopy(T* dst, long long ldd, long long sd, const T* src, long long lds, lo
             cudaStream_t st, const int* only = nullptr) {
   for (int b0 = 0; b0 < batch; b0 += 65535) {
     const int nb = (batch - b0 < 65535) ? batch - b0 : 65535;
-    dim3 grid((unsigned)exa_ceil_div(R * Cn, 256 * 4), (unsigned)nb);
+    dim3 grid(only ? 1u : (unsigned)exa_ceil_div(R * Cn, 256 * 4), (unsigned)nb);  // few of a subset have work
     submat_copy_kernel<T><<<grid, 256, 0, st>>>(dst + b0 * sd, ldd, sd, src + b0 * ss, lds, ss, R, Cn,
                                                 only ? only + b0 : nullptr);
     EXA_LAUNCH_CHECK();
@@ -1145,7 +1144,8 @@ int inverse_2x2(T* A, int n, long long stride, int batch, T* ws, long long sw, L
 // zero pivot or a non-finite entry, is inverted again from its original by the register kernel, which
 // pivots over all its rows.  Euler blocks (condition 380 to 2800, states perturbed by 1e-2): growth 1.0
 // at dtfactor 68, 1.4 at 1, with errors as from whole halves (2e-15); 6.9 at 0.1, where the leaves alone
-// lose a digit; 1e5 at 1e-6, where they leave two digits.
+// lose a digit; 1e5 at 1e-6, where they leave two digits.  Bound: one read of the blocks, 97 us per level
+// for 1000 halves of order 160 (0.36 GB); the assembly of 1000 such elements 12.58 -> 12.80 ms.
 constexpr int INV_LEAF = 96;
 constexpr double INV_GROWTH = 2.0;
 
@@ -1169,15 +1169,25 @@ __global__ void __launch_bounds__(256) inverse_growth_kernel(int n, int n1, cons
     if (!(v <= big)) bad = true;  // infinities and NaN
     else if (v > m[k]) m[k] = v;
   };
-  for (int t = tid; t < n * n; t += 256) {
-    const int r = t % n, c = t / n;
-    take(r >= n1 && c >= n1 ? 2 : 0, A[t]);
-  }
-  for (int t = tid; t < n1 * n1; t += 256) take(1, X[t]);
-  for (int t = tid; t < n2 * n2; t += 256) {
-    take(0, Y[t]);
-    take(3, O22[t % n2 + ldo * (t / n2)]);
-  }
+  // a column per warp, its entries in flight together (INV_MAX_N / 32 loads a lane)
+  auto block = [&](int k, const T* B, int rows, int c0, int c1, long long ld) {
+    for (int c = c0 + (tid >> 5); c < c1; c += 8) {
+      T v[INV_MAX_N / 32];
+#pragma unroll
+      for (int q = 0; q < INV_MAX_N / 32; ++q) {
+        const int r = (tid & 31) + 32 * q;
+        v[q] = r < rows ? B[r + ld * c] : T(0);
+      }
+#pragma unroll
+      for (int q = 0; q < INV_MAX_N / 32; ++q) take(k, v[q]);
+    }
+  };
+  block(0, A, n, 0, n1, n);
+  block(0, A, n1, n1, n, n);
+  block(2, A + n1, n2, n1, n, n);  // S
+  block(1, X, n1, 0, n1, n1);
+  block(0, Y, n2, 0, n2, n2);
+  block(3, O22, n2, 0, n2, ldo);
   __shared__ T red[8][4];
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
