@@ -165,8 +165,8 @@ __global__ void bbj_kernel(const BJob* jobs) {
   }
 }
 
-// Modified Gram-Schmidt, launch k of a step (the single-context sequence of exa_dot_partials,
-// mgs_step and mgs_finish, per job): k = 0 dots v_{i+1} with v_0; 1 <= k <= i subtracts h_{k-1}
+// Modified Gram-Schmidt, launch k of a step, vector by vector for each job (a context on its own takes
+// the triangular form of the same recurrence, exa_ortho.cu, which rounds differently): k = 0 dots v_{i+1} with v_0; 1 <= k <= i subtracts h_{k-1}
 // v_{k-1} and dots with v_k; k = i + 1 subtracts h_i v_i and takes |v_{i+1}|^2; k = i + 2 scales
 // v_{i+1} by 1 / h_{i+1}.  Jobs with i + 2 < k have nothing to do.
 __global__ void __launch_bounds__(VT) bmgs_kernel(const BJob* jobs, int k) {

@@ -346,9 +346,9 @@ int arnoldi_ops(ExaCtx& c, int i, const double* d_nrmb, double* d_relerr, double
 }
 
 // Enqueues Arnoldi step i.  Its first use runs the launches directly; from the second use on
-// the step is one CUDA graph, captured then and replayed after, which replaces some 30
-// launches (the matvec, the preconditioner, one Gram-Schmidt launch per basis vector, the
-// Givens update) by one.  The graph's arguments are fixed per context: the basis column,
+// the step is one CUDA graph, captured then and replayed after, which replaces the launches of
+// the matvec, the preconditioner and the Gram-Schmidt step with its Givens update (2 to 6 with
+// block Jacobi and modified Gram-Schmidt) by one.  The graph's arguments are fixed per context: the basis column,
 // the Hessenberg column, the residual slot.  Phase profiling records events between the
 // launches, so it runs the launches directly.  A capture that fails leaves the context on
 // direct launches.

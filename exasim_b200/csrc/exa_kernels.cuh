@@ -51,8 +51,6 @@ bool exa_vol_mat_tc_fits(const ExaDims& P);
 // trace component: row i + npe k, k = j + qk_group(npe) d) instead of B.
 int exa_k_vol_mat_tc(const ExaDims& P, const float* shapegw32, const UPacked& Sp, const double* rgJ, double* D,
                      double* B, const UPacked& Bp, int nb, int* flag, cudaStream_t st);
-// Block ILU(0) preconditioner on Cartesian sub-domains (Exasim preconditioner = 2): the
-// schedule built on the host (exa_bilu0.h) in device memory, and the sub-domain results.
 // The 1D tables of a tensor-product element: its shape tables, and its faces', are Kronecker
 // products of S (and D for the derivatives) with the first dimension fastest, at n1 nodes and n1
 // Gauss points per dimension; n1 = 0 where they are not.
@@ -65,6 +63,8 @@ struct ExaTensor {
 inline bool exa_tensor_blocks(const ExaDims& P, const ExaTensor& T) {
   return (P.nd == 2 || P.nd == 3) && T.n1 >= 3 && T.n1 <= 5;
 }
+// Block ILU(0) preconditioner on Cartesian sub-domains (Exasim preconditioner = 2): the
+// schedule built on the host (exa_bilu0.h) in device memory, and the sub-domain results.
 struct ExaSweepDev {
   int levels = 0;
   int *lev = nullptr, *row = nullptr, *ptr = nullptr, *blk = nullptr;

@@ -15,8 +15,9 @@
 // vectors up to OC_MAX_N entries run in one thread-block cluster that keeps w in registers (one
 // launch, partial sums through distributed shared memory), longer ones as three launches over the
 // GPU.  Every sum has a fixed partition and order, so results do not depend on scheduling.
-// Measured (B200, before: one launch per vector): 4800 unknowns, restart 50, 244 steps of a served
-// 2D solve 32.1 -> 8.3 ms in all; 553k unknowns, restart 50, 150 steps of an LDG solve 41.9 -> 23.5 ms.
+// Measured (B200, before: one launch per vector): 4800 unknowns, restart 50, 245 steps of a served
+// 2D solve 22.9 -> 5.2 ms for the call, with the face-by-face operator (face_op_kernel) at the same time;
+// 553k unknowns, restart 50, 150 steps of an LDG solve 41.9 -> 23.5 ms.
 #include <cooperative_groups.h>
 
 #include <algorithm>
