@@ -796,9 +796,9 @@ def run_served(args, device):
 QELIM_TRAFFIC_PER_ELEMENT = 2.326e9 / 1331
 # The same for the mixed form's q elimination: two 3xTF32 products (umma3_kernel, FP32 operands
 # split on chip), 0.564 and 0.642 GB read + written on the 10^3 mesh (the mean per launch), and the
-# trace rows (trace_q_kernel), 0.534 GB on the 9^3 mesh.
+# trace rows (trace_q_kernel), 0.761 GB there.
 QELIM_MIXED_TRAFFIC_PER_ELEMENT_LAUNCH = (0.564e9 + 0.642e9) / 1000 / 2
-TRACE_ROWS_TRAFFIC_PER_ELEMENT = 0.534e9 / 729
+TRACE_ROWS_TRAFFIC_PER_ELEMENT = 0.7605e9 / 1000
 
 
 def fp64_gemm_peak(torch):
@@ -903,7 +903,7 @@ def kernel_rooflines(s32, s64, mixed, plain, torch, steps):
                    "cp.async.bulk, split into TF32 hi and lo parts in shared memory)", q_ms - t_ms, 2 * q_regions,
                    qelim_products_bytes(sz) / 2, QELIM_MIXED_TRAFFIC_PER_ELEMENT_LAUNCH, "a 10^3")
     trace = hbm("trace_q_kernel (K += G MinvC, H -= G MinvE by sum factorization in FP32)", t_ms, t_regions,
-                trace_rows_bytes(sz), TRACE_ROWS_TRAFFIC_PER_ELEMENT, "a 9^3")
+                trace_rows_bytes(sz), TRACE_ROWS_TRAFFIC_PER_ELEMENT, "a 10^3")
     p_ms, p_regions, p_flops = plain["prof"]["qelim"]
     peak64 = fp64_gemm_peak(torch)
     pl = p_regions

@@ -105,7 +105,8 @@ __global__ void gemv_batch_kernel(GemmBatch g) {
 // Measured (B200; before: m8n8k4, 256 threads, 128 x 64 to 160 x 64 tiles, two CTAs per SM): 1000
 // products of 480 x 480 x 320 6.39 -> 5.57 ms (26.5 TFLOP/s of 37 that either mma shape reaches from
 // registers), of 320 x 480 x 320 3.89 -> 3.12 ms; 1331 of 125 x 125 x 375 724 -> 716 us.  ncu: the
-// tensor pipe is active 65 to 70% of the cycles, waits for copies and fixed latencies take the rest.
+// tensor pipe is active 65 to 70% of the cycles there, waits for copies and fixed latencies take the rest;
+// 51 and 33% in the products over 80 listed k (face_k), whose five chunks leave the start and the epilogue bare.
 // ----------------------------------------------------------------------------------
 constexpr int GK = 16, GST = 3, GSB = GK + 4;
 
