@@ -13,8 +13,10 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("model,n,p,precision", [("convdiff3d", 6, 4, 0), ("convdiff3d", 6, 4, 1), ("convdiff3d", 8, 2, 0),
                                                  ("convdiff3d", 3, 1, 0), ("euler3d", 4, 3, 0), ("euler3d", 4, 3, 1),
                                                  ("euler3d", 6, 2, 0), ("ns2d", 16, 3, 0), ("cdsin2d", 40, 4, 0),
-                                                 ("poisson2d", 24, 3, 0), ("poisson2d", 24, 3, 1)])
+                                                 ("poisson2d", 24, 3, 0), ("poisson2d", 24, 3, 1),
+                                                 ("ns2d_ilu", 16, 3, 0), ("euler3d_ldg", 6, 3, 0)])
 def test_estimate_covers_what_is_held(tmp_path, model, n, p, precision):
+    ilu, ldg, model = model.endswith("_ilu"), model.endswith("_ldg"), model.split("_")[0]
     B.build([model])
     d = str(tmp_path / "datain")
     if model == "poisson2d":
@@ -24,9 +26,9 @@ def test_estimate_covers_what_is_held(tmp_path, model, n, p, precision):
     elif model == "convdiff3d":
         cases.convdiff3d_hex(d, n=n, porder=p, nsteps=1)
     elif model == "ns2d":
-        cases.ns2d_tgv_quad(d, n=n, porder=p, nsteps=1, preconditioner=0)
+        cases.ns2d_tgv_quad(d, n=n, porder=p, nsteps=1, preconditioner=2 if ilu else 0)
     else:
-        cases.euler3d_vortex_hex(d, n=n, porder=p, nsteps=1)
+        cases.euler3d_vortex_hex(d, n=n, porder=p, nsteps=1, hybrid=0 if ldg else 1)
     blobs = read_datain(d)
     with Server(model, slots=1) as srv:
         srv.wait(srv.submit(blobs, precision=precision))
@@ -41,6 +43,8 @@ def test_estimate_covers_what_is_held(tmp_path, model, n, p, precision):
     # the mixed form has freed its FP64 blocks by now, which are part of what it needs at most
     m = ncf * (2 * nd if quad else 3)
     npe = (p + 1) ** nd if quad else (p + 1) * (p + 2) // 2
+    if ilu:  # face blocks: each face's own and those of the other faces of its elements, at most
+        slack += 8 * 2 * nf * ncf * ncf * (1 + 2 * (2 * nd - 1))
     if precision:
         slack += 8 * ne * m * (m + npe * ncu)
     print(model, n, p, precision, held >> 20, est >> 20, int(slack) >> 20)
