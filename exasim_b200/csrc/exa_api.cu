@@ -511,11 +511,14 @@ int exa_ctx_init(ExaCtx& c, const double* app, long long napp, const double* mas
   const size_t inv_ws = hdg ? exa_inverse_ws_size((int)n) : 0;
   const size_t vol_ws = (size_t)P.nge * P.nc + (size_t)P.nge * P.ncu + (size_t)P.nge * (P.nd + 1) * P.ncu;
   // with the q elimination by sum factorization neither B nor G is formed, but the face fluxes'
-  // derivatives with respect to q are kept (B is made when a caller asks for it: block_b)
+  // derivatives with respect to q are kept (B is made when a caller asks for it: block_b).  The chunk
+  // counts the mixed form's packed B all the same, so that its operands, about 0.5 MB per p = 4 hexahedron
+  // beside 0.45 MB of these arrays, do not outgrow the chunks with B and G (2 MB each in all).
   const bool qtp = hdg && exa_model_qelim_tp(P, c.tensor);
   const size_t bg = qtp ? 2 * (size_t)P.nfe * P.ngf * P.ncu * P.ncq : (n + m) * nqn;
   const size_t per_elem = hdg ? sizeof(double) * (n * n + n * m + m * n + bg +
-                                                  (size_t)P.nge * (P.nd + 1) * P.ncu * P.nc + n + inv_ws)
+                                                  (size_t)P.nge * (P.nd + 1) * P.ncu * P.nc + n + inv_ws) +
+                                    (qtp ? sizeof(float) * n * nqn : 0)
                               : sizeof(double) * (vol_ws + n);
   size_t cap = (size_t)8 << 30;
   c.neb = (int)std::max<size_t>(1, std::min<size_t>(std::min<size_t>(ne, cap / per_elem), 65535));
@@ -881,7 +884,7 @@ long long exa_ctx_estimate_bytes(const double* app, long long napp, const double
   const double bg = qtp ? 2.0 * P.nfe * P.ngf * ncu * P.ncq : (q ? (n + m) * npe * nd * ncu : 0.0);
   const double inv = hdg ? (double)exa_inverse_ws_size(P.n) : 0.0;
   // as exa_ctx_init: the element chunk
-  const double per = hdg ? n * n + 2 * n * m + bg + rg + n + inv : ug + n;
+  const double per = hdg ? n * n + 2 * n * m + bg + rg + n + inv + (qtp ? 0.5 * n * npe * nd * ncu : 0.0) : ug + n;
   const double nb = std::max(1.0, std::min(std::min(ne, std::floor((8LL << 30) / (8.0 * per))), 65535.0));
   // preconditioner blocks: block Jacobi one per face; block ILU(0) one per stored block of the
   // sub-domain face graph, at most the face itself and the other faces of its two elements
